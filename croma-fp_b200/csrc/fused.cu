@@ -21,7 +21,9 @@
 //      Nothing here depends on the evolving spectra (the eta cap aside, which
 //      then runs the chunk one segment at a time), so every segment of the
 //      snapshot is factored by one launch with full occupancy.
-//   2. steps_kernel, one warp per tracer: for each segment it loads the
+//   2. steps_packed_kernel (runs of 64 tracers and more): 16 rows a lane, the
+//      constants of a segment in registers and tensor memory; below that
+//      steps_kernel, one warp per tracer: for each segment it loads the
 //      factored rows (and the segment's source), and runs each sub-step as
 //      the two first-order linear recurrences of fp_thomas_solve_ws
 //      (src/fp_shared_core.c:226-257), each an affine warp scan: a local pass
@@ -43,7 +45,6 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 #include "croma_segment.cuh"
 
@@ -118,6 +119,7 @@ struct FusedParams {
     // instead of the resident ones and stops after cal_steps sub-steps
     double *cal_spec;
     int cal_steps;
+    const int *order;        // [nt] the packed steps kernel's tracer order within the chunk, or null (as they are)
 };
 
 __device__ __forceinline__ SegInfo segment_of(const FusedParams &P, int t, int slot)
@@ -1311,7 +1313,7 @@ __device__ __forceinline__ void substep_pcr(const Coef<SRC> &F, const double cc[
 // overlapping the forward scan), the warp scan with FP32 solves refined by
 // an FP64 residual, and warp PCR.
 enum { kSolveScan = 0, kSolveRefined = 1, kSolvePcr = 2, kSolveScanShared = 3, kSolveScanRhs = 4,
-       kSolveScan4 = 5 };
+       kSolveScan4 = 5, kSolvePacked = 6 };
 
 // Steps kernel: warp w of block b runs every segment [g0, g1) of tracer
 // t0 + b * WPB + w for species S with sub-step solver SOLVER.
@@ -1443,6 +1445,644 @@ __global__ void __launch_bounds__(WPB * 32,
     }
 #pragma unroll
     for (int r = 0; r < kR; r += 4) st4(Nrow + r, N + r);
+}
+
+// ---------------------------------------------------------------------------
+// Packed steps kernel: 16 rows a lane at every bin count, so NB / 16 lanes (8,
+// 16 or 32) run a tracer and a warp runs 4, 2 or 1 of them.
+//
+// What bounds a sub-step (measured on B200): a DFMA with three different
+// register operands takes 3 cycles of a scheduler, one that shares an operand
+// with the instruction before it 2.2, a DMUL or DADD 2; a dependent FP64
+// instruction waits 8; a 64-bit shuffle takes 25 and two cycles of the whole
+// SM.  A warp per tracer at 128 bins (4 rows a lane) spends more on its twelve
+// shuffles than on its arithmetic, and at 512 bins (16 rows) eight warps per
+// SM wait on their own chains.  So:
+//
+// * 16 rows a lane at 128 and 256 bins too: the scans of a sub-step serve
+//   four (two) tracers.
+// * The solve in block form.  Each lane solves its 16 rows with zero carries
+//   (forward chain, back chain); the solution is that plus the rows'
+//   responses to the two carries, x_r = raw_r + g_r cin + e_r cout, with
+//     c_r = h_0 .. h_r,  e_r = q_r .. q_15,  g_15 = c_15, g_r = c_r + q_r g_r+1
+//   constants of the segment.  cin is the exclusive scan of the forward
+//   chains' ends over the tracer's lanes, cout that of the back chains' ends
+//   plus g_0 cin.  The responses are independent rows sharing an operand.
+// * Both scans run under a chain.  While cout is still being scanned the next
+//   sub-step's forward chain runs on x without cout; its response to cout,
+//   E_r = e_r / d_r + h_r E_r-1, is added to the rows afterwards, during the
+//   forward scan and the back chain.
+// * The constants g, 1/d, E and dt src/d sit in tensor memory (96 or 128 of
+//   the 128 columns that a block of four warps holds) and are read a few rows
+//   ahead: tcgen05.ld is there after ~17 cycles, and the shared memory's
+//   bandwidth would not do.  N, h and q stay in registers.  That fits 168 of
+//   them: 12 warps per SM instead of 8.
+// * The next segment's rows come into shared memory by cp.async during the
+//   present one: all warps of an SM keep step, and would ask for 190 KB at once.
+//
+// All terms are nonnegative (an M-matrix, nonnegative spectra), so nothing
+// cancels and the error is the two-pass form's.
+//
+// Measured, whole kernel with its segment switches, before (a warp per tracer)
+// and now: 131,072 tracers x 500 sub-steps of 128 bins 8.20 -> 4.42 ms, of 512
+// bins 24.6 -> 20.6 ms (with a source 25.4 -> 21.3), 65,536 of 256 bins 6.24 ->
+// 5.2 ms; 30,011 with 11 to 500 sub-steps 0.60 -> 0.25 ms; 64 tracers 152 ->
+// 131 us.  FP64 pipe 52 % (its operand reads ~70 %), stalls per issue:
+// dependent FP64 1.9, shuffles and tensor memory 0.7 to 1.2.
+constexpr int kPkRows = 16;
+constexpr int kPkLanes = NB / kPkRows;    // lanes per tracer
+constexpr int kPkTracers = 32 / kPkLanes; // tracers per warp
+constexpr int kPkWarps = 4;               // one per TMEM lane quarter
+constexpr int kPkColumns = 128;           // TMEM columns of a block: 3 blocks per SM hold 384 of 512
+
+__device__ __forceinline__ double pk_up(double v, int d) { return __shfl_up_sync(kFull, v, d, kPkLanes); }
+__device__ __forceinline__ double pk_down(double v, int d) { return __shfl_down_sync(kFull, v, d, kPkLanes); }
+
+// Sixteen (eight) 32-bit TMEM columns of the warp's lanes.  The loads are
+// asynchronous: the registers are valid after tmem_wait, which names them so
+// that no use is scheduled before it (tmem_after8: a further load that the same
+// wait covers).
+struct Tmem16 {
+    unsigned r[16];
+    __device__ __forceinline__ double d(int i) const { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
+};
+__device__ __forceinline__ void tmem_ld16(unsigned t, Tmem16 &u)
+{
+    unsigned *r = u.r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(t));
+}
+__device__ __forceinline__ void tmem_ld8(unsigned t, unsigned *r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(t));
+}
+__device__ __forceinline__ void tmem_wait(Tmem16 &u)
+{
+    unsigned *r = u.r;
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
+}
+__device__ __forceinline__ void tmem_after8(unsigned *r)
+{
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+}
+__device__ __forceinline__ void tmem_wait8(unsigned *r)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+}
+__device__ __forceinline__ void tmem_st8(unsigned t, const unsigned *r)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void pk_set(unsigned *r, int i, double v)
+{
+    r[2 * i] = (unsigned)__double2loint(v);
+    r[2 * i + 1] = (unsigned)__double2hiint(v);
+}
+__device__ __forceinline__ double pk_get(const unsigned *r, int i) { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
+
+// TMEM columns of the four rows of chunk k: their (g, 1/d) pairs, their E,
+// their dt src/d.
+__device__ __forceinline__ unsigned pk_fwd(unsigned tm, int k) { return tm + k * 16; }
+__device__ __forceinline__ unsigned pk_resp(unsigned tm, int k) { return tm + 64 + k * 8; }
+__device__ __forceinline__ unsigned pk_src(unsigned tm, int k) { return tm + 96 + k * 8; }
+
+// The walk of each lane's tracer through its runs of sub-steps, kept in
+// shared memory (each lane its own copy): it is touched once a run, and in
+// registers it would push the sub-step's constants out of theirs.
+constexpr int kPkThreads = kPkWarps * 32;
+struct PkWalk {
+    int tl[kPkThreads];      // tracer within the chunk
+    int gi[kPkThreads];      // segment
+    int run[kPkThreads];     // run within the segment: before, inside, after the Dpp window
+    int rem[kPkThreads];     // sub-steps left in the run; < 0: no run left
+    int sl[kPkThreads], el[kPkThreads], steps[kPkThreads];
+    int pgi[kPkThreads], pset[kPkThreads];   // segment and set whose rows the row buffer holds
+    double dt[kPkThreads];
+};
+// The next segment's scalars of each group (the last 16 bytes of its SegPre, and dt).
+struct PkNext {
+    int4 meta[kPkWarps * kPkTracers];   // flags, sl, el, steps
+    double dt[kPkWarps * kPkTracers];
+};
+static_assert(offsetof(SegPre, flags) % 16 == 0 && offsetof(SegPre, steps) == offsetof(SegPre, flags) + 12 &&
+                  sizeof(SegPre) % 16 == 0 && offsetof(SegPre, dt) % 8 == 0,
+              "the packed steps kernel copies flags .. steps as 16 bytes");
+
+// Row buffer of a warp: the arrays 1/d, a/d, c/d (and the source) of its
+// groups' next run, 512 doubles each, filled by cp.async while the present
+// run's sub-steps go on.  Without it all warps of an SM, which keep step, ask
+// for their rows at once at each segment: 190 KB an SM, 12 % of the kernel's
+// time at 512 bins.  Copies are contiguous across the lanes; 16-byte piece c
+// of a group's array (owner lane c / 8) sits at c ^ (owner & 7), so that the
+// lanes' reads of their own 128 bytes meet no bank twice.
+__device__ __forceinline__ int pk_piece(int c) { return c ^ ((c >> 3) & 7); }
+
+template <int S, bool SRC>
+__device__ __forceinline__ void pk_fetch(const FusedParams &P, double *buf, int gi, int set, int tl, int gl)
+{
+    const double *f = fac_ptr(P, S, gi, set, tl);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int c = i * kPkLanes + gl;
+#pragma unroll
+        for (int k = 0; k < 3; k++) cp_async16(buf + k * 512 + 2 * pk_piece(c), f + k * NB + 2 * c, true);
+    }
+    if (SRC) {
+        const double *src = (S == 1 && P.inje) ? P.inje + ((size_t)gi * P.nt + tl) * NB
+                                               : (S == 0 ? P.a.qpi : P.a.qepri) + (size_t)(P.t0 + tl) * NB;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int c = i * kPkLanes + gl;
+            cp_async16(buf + 3 * 512 + 2 * pk_piece(c), src + 2 * c, true);
+        }
+    }
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// the lane's 16 rows of array k
+__device__ __forceinline__ void pk_read(const double *buf, int k, int gl, double v[kPkRows])
+{
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const double2 x = *reinterpret_cast<const double2 *>(buf + k * 512 + 2 * pk_piece(gl * 8 + j));
+        v[2 * j] = x.x;
+        v[2 * j + 1] = x.y;
+    }
+}
+
+// Species S of the chunk's tracers, every segment [g0, g1).  Tracers come in
+// the chunk's order (P.order: by falling sub-step count, so that the tracers
+// of a warp and of a block end together); each group of kPkLanes lanes walks
+// its own tracer's runs of sub-steps (the segments, split by the Dpp window)
+// and the warp advances all its groups by the smallest remaining run.  When
+// any group starts a run, all load their constants again (the others' are
+// what they were).  A group without work holds the identity (1/d = 1, the
+// rest 0), which leaves its rows as they are, bit for bit.
+template <int S, bool SRC>
+__global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams P)
+{
+    constexpr int R = kPkRows;
+    extern __shared__ double4 steps_smem[];
+    __shared__ unsigned tmem_base;
+    __shared__ PkWalk walk_smem;
+    __shared__ PkNext next;
+    volatile PkWalk &walk = walk_smem;
+    const int me = threadIdx.x, w = me >> 5, gl = me & (kPkLanes - 1);
+    if (w == 0) {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(&tmem_base);
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "n"(kPkColumns)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    __syncthreads();
+    const unsigned tm = tmem_base + ((unsigned)(w * 32) << 16);   // the warp's lane quarter
+    double N[R], h[R], q[R];
+    double cin = 0.0, b = 0.0;   // the forward carry, the back chain's end
+    {
+        const int pos = (blockIdx.x * kPkWarps + w) * kPkTracers + (me & 31) / kPkLanes;
+        const bool mine = pos < P.nt;
+        const int tl = mine ? (P.order ? P.order[pos] : pos) : -1;
+        walk.tl[me] = tl;
+        walk.gi[me] = -1;
+        walk.run[me] = 2;
+        walk.rem[me] = mine ? 0 : -1;
+        walk.pgi[me] = -1;
+        const double *row = (S == 0 ? P.a.crp : P.a.cre) + (size_t)(P.t0 + max(tl, 0)) * NB + gl * R;
+#pragma unroll
+        for (int r = 0; r < R; r++) N[r] = 0.0;
+        if (mine) {
+#pragma unroll
+            for (int r = 0; r < R; r += 4) ld4(row + r, N + r);
+        }
+    }
+#pragma unroll 1
+    for (;;) {
+        const int group = me / kPkLanes;
+        double *buf = reinterpret_cast<double *>(steps_smem) + (size_t)w * (SRC ? 4 : 3) * 512 +
+                      (group % kPkTracers) * NB;
+        bool load = walk.rem[me] >= 0;   // the group has work
+        int want = 0;                    // its coefficient set
+        cp_async_wait_all();             // the rows and scalars fetched for the next run
+        __syncwarp();
+        {
+            const int tl = max(walk.tl[me], 0), nslot = P.g1 - P.g0;
+            int k = walk.run[me];
+            if (walk.rem[me] == 0) {     // the next run of a group that has none
+                int gi = walk.gi[me], rem = 0, sl = walk.sl[me], el = walk.el[me], steps = walk.steps[me];
+#pragma unroll 1
+                while (rem <= 0) {
+                    if (k < 2) {
+                        k++;
+                    } else {
+                        if (++gi >= nslot) {
+                            rem = -1;
+                            break;
+                        }
+                        int4 mt;
+                        if (gi > 0) {
+                            mt = next.meta[group];
+                            walk.dt[me] = next.dt[group];
+                        } else {
+                            const SegPre *__restrict__ pre = P.pre + tl;
+                            mt = make_int4(pre->flags, pre->sl, pre->el, pre->steps);
+                            walk.dt[me] = pre->dt;
+                        }
+                        if (!(mt.x & kPreActive)) {   // a tracer's active segments come first
+                            rem = -1;
+                            break;
+                        }
+                        steps = mt.w;
+                        sl = (mt.x & kPreWindowed) ? min(max(mt.y, 0), steps) : 0;
+                        el = (mt.x & kPreWindowed) ? min(max(mt.z, sl), steps) : steps;
+                        k = 0;
+                        if (S == 0 && P.np_seg) {
+                            double *o = P.np_seg + ((size_t)gi * P.nt + tl) * NB + gl * R;
+#pragma unroll
+                            for (int r = 0; r < R; r += 4) st4_cg(o + r, N + r);
+                        }
+                    }
+                    rem = (k == 0) ? sl : (k == 1 ? el - sl : steps - el);
+                }
+                if (rem > 0 && k != 1 && P.sets < 2) {   // no off set in the workspace: report, leave N as it was
+                    if (gl == 0) atomicOr(P.a.err, kErrBadInput);
+                    rem = -1;
+                }
+                load = rem > 0;
+                walk.gi[me] = gi;
+                walk.run[me] = k;
+                walk.rem[me] = rem;
+                walk.sl[me] = sl;
+                walk.el[me] = el;
+                walk.steps[me] = steps;
+            }
+            want = (k == 1) ? 0 : 1;
+        }
+        __syncwarp();
+        if (!__any_sync(kFull, load)) break;
+        const bool miss = load && (walk.pgi[me] != walk.gi[me] || walk.pset[me] != want);
+        if (__any_sync(kFull, miss)) {
+            if (miss) pk_fetch<S, SRC>(P, buf, walk.gi[me], want, walk.tl[me], gl);
+            cp_async_wait_all();
+            __syncwarp();
+        }
+        // the constants of the run: h and q to registers, g, E, 1/d and the
+        // source to TMEM, the scan multipliers
+        double hk[5], qk[5];
+        {
+            double iv[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                iv[r] = 1.0;
+                h[r] = q[r] = 0.0;
+            }
+            if (load) {
+                pk_read(buf, 0, gl, iv);
+                if (SRC) pk_read(buf, 3, gl, h);
+            }
+            if (SRC) {
+                const double dt = walk.dt[me];
+                __syncwarp();
+#pragma unroll
+                for (int kk = 0; kk < R / 4; kk++) {
+                    unsigned u[8];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) pk_set(u, i, load ? (dt * h[4 * kk + i]) * iv[4 * kk + i] : 0.0);
+                    tmem_st8(pk_src(tm, kk), u);
+                }
+            }
+            if (load) {
+                pk_read(buf, 1, gl, h);
+                pk_read(buf, 2, gl, q);
+                if (gl == 0) h[0] = 0.0;
+                if (gl == kPkLanes - 1) q[R - 1] = 0.0;
+            }
+            __syncwarp();   // the buffer is read
+            if (load) {
+                // the rows of the next run (another set of this segment, or
+                // the next one's first run, taken to be of the set this one
+                // ends with) and the scalars of the next segment
+                const int gi = walk.gi[me], k = walk.run[me], tl = walk.tl[me];
+                const int sl = walk.sl[me], el = walk.el[me], steps = walk.steps[me];
+                int pgi = gi, pset = 0;
+                if (k == 0 && el > sl) pset = 0;
+                else if (k < 2 && steps > el) pset = 1;
+                else {
+                    pgi = gi + 1;
+                    pset = (steps > el || el == sl) ? 1 : 0;
+                }
+                if (pgi < P.g1 - P.g0) pk_fetch<S, SRC>(P, buf, pgi, pset, tl, gl);
+                else pgi = -1;
+                walk.pgi[me] = pgi;
+                walk.pset[me] = pset;
+                if (gl == 0 && gi + 1 < P.g1 - P.g0) {
+                    const SegPre *pre = P.pre + (size_t)(gi + 1) * P.nt + tl;
+                    cp_async16(&next.meta[group], &pre->flags, true);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                     (unsigned)__cvta_generic_to_shared(&next.dt[group])),
+                                 "l"(&pre->dt)
+                                 : "memory");
+                }
+            }
+            // e, then E = 1/d e + h E_r-1 (upwards)
+            double v[R], H = 1.0, Q = 1.0;
+#pragma unroll
+            for (int r = R - 1; r >= 0; r--) {
+                Q *= q[r];
+                v[r] = iv[r] * Q;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int kk = 0; kk < R / 4; kk++) {
+                unsigned u[8];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * kk + i;
+                    if (r > 0) v[r] = fma(h[r], v[r - 1], v[r]);
+                    pk_set(u, i, v[r]);
+                }
+                tmem_st8(pk_resp(tm, kk), u);
+            }
+            // c, then g = c + q g_r+1 (downwards)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                H *= h[r];
+                v[r] = H;
+            }
+#pragma unroll
+            for (int r2 = R / 2 - 1; r2 >= 0; r2--) {
+                unsigned u[8];
+#pragma unroll
+                for (int i = 1; i >= 0; i--) {
+                    const int r = 2 * r2 + i;
+                    if (r < R - 1) v[r] = fma(q[r], v[r + 1], v[r]);
+                    pk_set(u, 2 * i, v[r]);
+                    pk_set(u, 2 * i + 1, iv[r]);
+                }
+                tmem_st8(pk_fwd(tm, r2 / 2) + 8 * (r2 & 1), u);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int lv = 0; (1 << lv) < kPkLanes; lv++) {
+                const int off = 1 << lv;
+                hk[lv] = gl >= off ? H : 0.0;
+                qk[lv] = gl + off < kPkLanes ? Q : 0.0;
+                const double Hu = pk_up(H, off), Qd = pk_down(Q, off);
+                H *= gl >= off ? Hu : 1.0;
+                Q *= gl + off < kPkLanes ? Qd : 1.0;
+            }
+        }
+        int m = load ? walk.rem[me] : 0x7fffffff;
+#pragma unroll
+        for (int off = 16; off >= kPkLanes; off >>= 1) m = min(m, __shfl_xor_sync(kFull, m, off));
+        __syncwarp();
+        // m sub-steps of every group.  At the group's ends the shuffles return
+        // the lane's own value, whose responses are zero (h of the first row,
+        // q of the last).
+        constexpr int kLevels = kPkLanes == 8 ? 3 : (kPkLanes == 16 ? 4 : 5);
+        double cout = 0.0;
+        Tmem16 U;            // (g, 1/d) of four rows
+        unsigned V[8];       // dt src/d of four rows
+        unsigned W[2][8];    // E of four rows
+        tmem_ld16(pk_fwd(tm, 0), U);
+        if (SRC) tmem_ld8(pk_src(tm, 0), V);
+#pragma unroll 1
+        for (int go = m; go > 0; go--) {
+            // forward chain of the rows without cout, under the back scan
+            double s = 0.0;
+#pragma unroll
+            for (int kk = 0; kk < R / 4; kk++) {
+                tmem_wait(U);
+                if (SRC) tmem_after8(V);
+                if (kk == 0) b = fma(U.d(0), cin, b);   // the back chain's end and its response to cin, g_0
+                const double t = kk < kLevels ? pk_down(b, 1 << kk) : 0.0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * kk + i;
+                    N[r] = fma(U.d(2 * i), cin, N[r]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * kk + i;
+                    N[r] = SRC ? fma(N[r], U.d(2 * i + 1), pk_get(V, i)) : N[r] * U.d(2 * i + 1);
+                }
+                if (kk < R / 4 - 1) {
+                    tmem_ld16(pk_fwd(tm, kk + 1), U);
+                    if (SRC) tmem_ld8(pk_src(tm, kk + 1), V);
+                } else {
+                    tmem_ld8(pk_resp(tm, 3), W[1]);
+                    tmem_ld8(pk_resp(tm, 2), W[0]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * kk + i;
+                    s = fma(h[r], s, N[r]);
+                    N[r] = s;
+                }
+                if (kk < kLevels) b = fma(qk[kk], t, b);
+            }
+            if (kLevels > 4) b = fma(qk[4], pk_down(b, 16), b);
+            cout = pk_down(b, 1);
+            // the rows' responses to cout and the back chain, under the forward scan
+            tmem_wait8(W[1]);
+            tmem_after8(W[0]);
+            s = fma(pk_get(W[1], 3), cout, s);
+            b = 0.0;
+#pragma unroll
+            for (int kk = R / 4 - 1; kk >= 0; kk--) {
+                unsigned *E = W[kk & 1];
+                if (kk < R / 4 - 2) tmem_wait8(E);
+                const double t = R / 4 - 1 - kk < kLevels ? pk_up(s, 1 << (R / 4 - 1 - kk)) : 0.0;
+#pragma unroll
+                for (int i = 3; i >= 0; i--) {
+                    const int r = 4 * kk + i;
+                    N[r] = fma(pk_get(E, i), cout, N[r]);
+                }
+                if (kk >= 2) {
+                    tmem_ld8(pk_resp(tm, kk - 2), W[kk & 1]);
+                } else if (kk == 0) {
+                    tmem_ld16(pk_fwd(tm, 0), U);
+                    if (SRC) tmem_ld8(pk_src(tm, 0), V);
+                }
+#pragma unroll
+                for (int i = 3; i >= 0; i--) {
+                    const int r = 4 * kk + i;
+                    b = fma(q[r], b, N[r]);
+                    N[r] = b;
+                }
+                if (R / 4 - 1 - kk < kLevels) s = fma(hk[R / 4 - 1 - kk], t, s);
+            }
+            if (kLevels > 4) s = fma(hk[4], pk_up(s, 16), s);
+            cin = pk_up(s, 1);
+        }
+        tmem_wait(U);
+        if (SRC) tmem_after8(V);
+        // where the run ends, the last sub-step's responses: x = raw + g cin +
+        // e cout; the other groups go on from their raw rows, so that no
+        // result depends on which tracers share a warp
+        const int left = load ? walk.rem[me] - m : 0;
+        const bool done = kPkTracers == 1 || left == 0;
+        double bb = fma(U.d(0), cin, b);
+#pragma unroll
+        for (int lv = 0; lv < kLevels; lv++) bb = fma(qk[lv], pk_down(bb, 1 << lv), bb);
+        cout = pk_down(bb, 1);
+#pragma unroll
+        for (int r = R - 1; r >= 0; r--) {
+            cout *= q[r];   // e_r cout
+            N[r] = done ? N[r] + cout : N[r];
+        }
+#pragma unroll
+        for (int kk = 0; kk < R / 4; kk++) {
+            tmem_ld16(pk_fwd(tm, kk), U);
+            tmem_wait(U);
+#pragma unroll
+            for (int i = 0; i < 4; i++) N[4 * kk + i] = done ? fma(U.d(2 * i), cin, N[4 * kk + i]) : N[4 * kk + i];
+        }
+        cin = done ? 0.0 : cin;
+        b = done ? 0.0 : b;
+        if (load) walk.rem[me] = left;
+    }
+    if (walk.tl[me] >= 0) {
+        double *row = (S == 0 ? P.a.crp : P.a.cre) + (size_t)(P.t0 + walk.tl[me]) * NB + gl * R;
+#pragma unroll
+        for (int r = 0; r < R; r += 4) st4(row + r, N + r);
+    }
+    __syncthreads();
+    if (w == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kPkColumns));
+}
+
+template <int S, bool SRC>
+cudaError_t launch_packed(cudaStream_t st, const FusedParams &P)
+{
+    constexpr size_t smem = (size_t)kPkWarps * (SRC ? 4 : 3) * 512 * sizeof(double);
+    static const cudaError_t attr = cudaFuncSetAttribute(steps_packed_kernel<S, SRC>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess) return attr;
+    const int per = kPkWarps * kPkTracers;
+    steps_packed_kernel<S, SRC><<<(P.nt + per - 1) / per, kPkThreads, smem, st>>>(P);
+    return cudaGetLastError();
+}
+
+// Order of the chunk's tracers for the packed steps kernel: by falling
+// sub-step count, in bins a sixteenth of an octave wide (exact below 32), the
+// order within a bin left open -- no tracer's result depends on which tracers
+// share its warp, only the time does.  One block up to kOrderOneBlock tracers;
+// beyond, the counts (order_count_kernel) and then the places, each block
+// reserving its range of a bin with one atomic.
+constexpr int kOrderBins = 288;
+constexpr int kOrderOneBlock = 4096;
+constexpr int kOrderThreads = 1024;
+
+__device__ __forceinline__ int order_bin(int nsub)   // 0 = most sub-steps
+{
+    int b = nsub;
+    if (nsub >= 32) {
+        const int e = 31 - __clz(nsub);   // >= 5; nsub <= 1e6 gives e <= 19
+        b = 32 + (min(e, 19) - 5) * 16 + ((nsub >> (e - 4)) & 15);
+    }
+    return kOrderBins - 1 - max(0, min(b, kOrderBins - 1));
+}
+
+// exclusive prefix of the bins in place (all threads call it)
+__device__ __forceinline__ void order_prefix(unsigned *bins)
+{
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        unsigned carry = 0;
+        for (int b0 = 0; b0 < kOrderBins; b0 += 32) {
+            const unsigned v = bins[b0 + threadIdx.x];
+            unsigned s = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned o = __shfl_up_sync(kFull, s, off);
+                if ((int)threadIdx.x >= off) s += o;
+            }
+            bins[b0 + threadIdx.x] = carry + s - v;
+            carry += __shfl_sync(kFull, s, 31);
+        }
+    }
+    __syncthreads();
+}
+
+// one atomic per bin and warp: most tracers of a run have the same count
+__device__ __forceinline__ unsigned order_take(unsigned *bins, int b, bool on)
+{
+    const unsigned peers = __match_any_sync(kFull, on ? b : -1);
+    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+    unsigned base = 0;
+    if (on && lane == leader) base = atomicAdd(bins + b, (unsigned)__popc(peers));
+    base = __shfl_sync(kFull, base, leader);
+    return base + __popc(peers & ((1u << lane) - 1u));
+}
+
+__global__ void __launch_bounds__(kOrderThreads) order_one_kernel(int nt, const int *nsub, int *order)
+{
+    __shared__ unsigned bins[kOrderBins];
+    for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) bins[b] = 0;
+    __syncthreads();
+    const int top = (nt + 31) & ~31;
+    for (int i = threadIdx.x; i < top; i += blockDim.x) order_take(bins, i < nt ? order_bin(nsub[i]) : 0, i < nt);
+    order_prefix(bins);
+    for (int i = threadIdx.x; i < top; i += blockDim.x) {
+        const unsigned p = order_take(bins, i < nt ? order_bin(nsub[i]) : 0, i < nt);
+        if (i < nt) order[p] = i;
+    }
+}
+
+// counts of the bins in bins[0 .. kOrderBins), zeroed before the launch
+__global__ void __launch_bounds__(kOrderThreads) order_count_kernel(int nt, const int *nsub, unsigned *bins)
+{
+    __shared__ unsigned mine[kOrderBins];
+    for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) mine[b] = 0;
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    order_take(mine, i < nt ? order_bin(nsub[i]) : 0, i < nt);
+    __syncthreads();
+    for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x)
+        if (mine[b]) atomicAdd(bins + b, mine[b]);
+}
+
+// bins: the counts, then kOrderBins cursors (zeroed before the count)
+__global__ void __launch_bounds__(kOrderThreads) order_place_kernel(int nt, const int *nsub, unsigned *bins, int *order)
+{
+    __shared__ unsigned first[kOrderBins], mine[kOrderBins];
+    for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) {
+        first[b] = bins[b];
+        mine[b] = 0;
+    }
+    order_prefix(first);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = i < nt ? order_bin(nsub[i]) : 0;
+    const unsigned at = order_take(mine, b, i < nt);
+    __syncthreads();
+    for (int c = threadIdx.x; c < kOrderBins; c += blockDim.x)
+        if (mine[c]) first[c] += atomicAdd(bins + kOrderBins + c, mine[c]);
+    __syncthreads();
+    if (i < nt) order[first[b] + at] = i;
+}
+
+cudaError_t launch_order(cudaStream_t st, int nt, const int *nsub, unsigned *bins, int *order)
+{
+    if (nt <= kOrderOneBlock) {
+        order_one_kernel<<<1, kOrderThreads, 0, st>>>(nt, nsub, order);
+        return cudaGetLastError();
+    }
+    const cudaError_t e = cudaMemsetAsync(bins, 0, 2 * kOrderBins * sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    const int blocks = (nt + kOrderThreads - 1) / kOrderThreads;
+    order_count_kernel<<<blocks, kOrderThreads, 0, st>>>(nt, nsub, bins);
+    order_place_kernel<<<blocks, kOrderThreads, 0, st>>>(nt, nsub, bins, order);
+    return cudaGetLastError();
 }
 
 // Per-step kernel (the plain path): warp w of block b advances tracer
@@ -1761,10 +2401,11 @@ cudaError_t launch_steps_variant(cudaStream_t st, const FusedParams &P, int trac
 
 // Variants the autotuner chooses between: (solver, warps per block).
 constexpr int kStepVariants = CROMA_B200_STEPS_VARIANTS;
-constexpr int kVariantSolver[kStepVariants] = {kSolveScan, kSolveScan, kSolveScanShared, kSolveScanShared,
-                                               kSolvePcr, kSolveScanRhs, kSolveScanRhs, kSolveScan4,
-                                               kSolveScan4};
-constexpr int kVariantWpb[kStepVariants] = {1, 2, 1, 2, 1, 1, 2, 1, 2};
+constexpr int kPackedVariant = kStepVariants;   // the packed kernel: by rule (packed_rule), never tuned
+constexpr int kVariantSolver[kStepVariants + 1] = {kSolveScan, kSolveScan, kSolveScanShared, kSolveScanShared,
+                                                   kSolvePcr, kSolveScanRhs, kSolveScanRhs, kSolveScan4,
+                                                   kSolveScan4, kSolvePacked};
+constexpr int kVariantWpb[kStepVariants + 1] = {1, 2, 1, 2, 1, 1, 2, 1, 2, kPkWarps * kPkTracers};
 
 // Arithmetic families: variants of one family compute bit-identical results
 // (the same operations in the same order; only where the constants live and
@@ -1807,23 +2448,16 @@ int tridiag_env()
     return 0;
 }
 
-// The autotuner: on the first chunk a context evolves, each admissible
-// variant of the family tune_family names runs the chunk's first tracers (at
-// most kTuneTracers) for their first 16 sub-steps on a copy of their spectra,
-// timed with CUDA events; the fastest is kept for the context's species.  Results are recorded in
-// ctx.tune.  kTuneTracers is several full waves of every variant (8 to 24
-// warps per SM on 148 SMs): a sample below one wave favours the variants
-// with more warps per SM, which lose at full size.  A calibration on the full
-// sample is kept for the process (per species, source and
-// CROMA_CUDA_TRIDIAG setting) and reused by later contexts with at least as
-// many tracers; smaller chunks calibrate on themselves.
-// CROMA_B200_STEPS_VARIANT = 0..8 fixes the variant (scan x1, scan x2, shared
-// scan x1, shared scan x2, PCR, rhs-shared scan x1, rhs-shared scan x2,
-// short-chain scan x1, short-chain scan x2)
-// without calibrating, for reproducible profiles; unset or out of range: tune.
+// The autotuner of runs below the packed kernel's line (and of PCR): on the
+// first chunk a context evolves, each admissible variant of the family
+// tune_family names runs the chunk's tracers (at most kTuneTracers) for their
+// first 16 sub-steps on a copy of their spectra, timed with CUDA events; the
+// fastest is kept for the context's species.  Results are recorded in
+// ctx.tune.  CROMA_B200_STEPS_VARIANT = 0..8 fixes the variant (scan x1, scan
+// x2, shared scan x1, shared scan x2, PCR, rhs-shared scan x1, rhs-shared scan
+// x2, short-chain scan x1, short-chain scan x2) without calibrating, for
+// reproducible profiles; unset or out of range: tune.
 constexpr int kTuneTracers = 16384;
-TuneState g_tune[2][2][3];   // [species][source][CROMA_CUDA_TRIDIAG: unset, thomas, pcr]
-std::mutex g_tune_mu;
 
 int fixed_variant_env()
 {
@@ -1831,6 +2465,21 @@ int fixed_variant_env()
     if (!e || !*e) return -1;
     const int v = atoi(e);
     return (v >= 0 && v < kStepVariants) ? v : -1;
+}
+
+// Which runs take the packed kernel: all of the FP64 on-chip path from
+// kPackedMin tracers on, unless the environment asks for PCR or names a
+// variant.  The line is on the run's tracers, not the chunk's, so that no
+// result depends on how a run is cut into chunks.  At the line the packed
+// kernel gains 14 % of the sub-steps' time (128 bins, 64 tracers: 152 -> 131
+// us) and spares the calibration's launches and waits; below it a launch is a
+// few blocks that wait on one warp's chain in either form, and the tuned
+// variants, which the environment can still name, stay.
+constexpr int kPackedMin = 64;
+bool packed_rule(const Context &ctx, const FusedParams &P)
+{
+    return ctx.cfg.path == CROMA_PATH_FUSED && P.a.ntracer >= kPackedMin && fixed_variant_env() < 0 &&
+           tridiag_env() != 2;
 }
 
 template <int S>
@@ -1845,15 +2494,6 @@ int tune_steps(Context &ctx, const FusedParams &P, bool src)
     }
     const int env = tridiag_env();
     const int T = min(P.nt, kTuneTracers), steps = 16;
-    TuneState *shared = nullptr;
-    if (T == kTuneTracers) {
-        shared = &g_tune[S][src ? 1 : 0][env];
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        if (shared->tuned) {
-            tu = *shared;
-            return 0;
-        }
-    }
     double *scratch = nullptr;
     CROMA_CUDA(dev_alloc(ctx, &scratch, (size_t)T * NB * sizeof(double)));
     struct Free {
@@ -1894,10 +2534,6 @@ int tune_steps(Context &ctx, const FusedParams &P, bool src)
     tu.tuned = 1;
     tu.tracers = T;
     tu.steps = steps;
-    if (shared) {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        if (!shared->tuned) *shared = tu;
-    }
     return 0;
 }
 
@@ -1914,7 +2550,16 @@ cudaError_t launch_steps(Context &ctx, const FusedParams &P, bool src, bool pers
         if (src) return launch_steps_variant<S, true, kSolveRefined, 1>(ctx.stream, P, 0);
         return launch_steps_variant<S, false, kSolveRefined, 1>(ctx.stream, P, 0);
     }
-    if (!ctx.tune[S].tuned) {
+    if (packed_rule(ctx, P)) {
+        TuneState &tu = ctx.tune[S];
+        if (tu.variant != kPackedVariant) {
+            tu = TuneState{};
+            tu.variant = kPackedVariant;
+        }
+        tu.tuned = 1;
+        return src ? launch_packed<S, true>(ctx.stream, P) : launch_packed<S, false>(ctx.stream, P);
+    }
+    if (!ctx.tune[S].tuned || ctx.tune[S].variant == kPackedVariant) {
         const int rc = tune_steps<S>(ctx, P, src);
         if (rc) return cudaErrorUnknown;
     }
@@ -1963,7 +2608,7 @@ WorkspaceShape workspace_shape(const ModelParams &mp, int cap, double workspace_
 double fused_workspace_bytes(const ModelParams &mp, int cap, double workspace_cap, int path)
 {
     const WorkspaceShape w = workspace_shape(mp, cap, workspace_cap, path == CROMA_PATH_PLAIN);
-    return (double)w.chunk * w.per_tracer + 8.0 * cap;
+    return (double)w.chunk * (w.per_tracer + sizeof(int)) + 8.0 * cap + 2.0 * kOrderBins * sizeof(unsigned);
 }
 
 int fused_reserve(Context &ctx, int cap)
@@ -1977,9 +2622,11 @@ int fused_reserve(Context &ctx, int cap)
     dev_free(ctx, ctx.d_np_seg);
     dev_free(ctx, ctx.d_segpre);
     dev_free(ctx, ctx.d_work);
+    dev_free(ctx, ctx.d_order);
     ctx.d_inje = ctx.d_eta_scale = ctx.d_fac = ctx.d_np_seg = nullptr;
     ctx.d_segpre = nullptr;
     ctx.d_work = nullptr;
+    ctx.d_order = nullptr;
     ctx.fused_chunk = ctx.fused_nseg = ctx.fused_sets = 0;
     const size_t rows = (size_t)nseg * chunk * NB;
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_fac, (size_t)2 * sets * rows * 3 * sizeof(double)));
@@ -1988,6 +2635,7 @@ int fused_reserve(Context &ctx, int cap)
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_eta_scale, (size_t)cap * sizeof(double)));
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_segpre, (size_t)nseg * chunk * sizeof(SegPre)));
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_work, 2 * sizeof(unsigned)));
+    CROMA_CUDA(dev_alloc(ctx, &ctx.d_order, (2 * kOrderBins + (size_t)chunk) * sizeof(int)));
     ctx.fused_chunk = (int)chunk;
     ctx.fused_nseg = nseg;
     ctx.fused_sets = sets;
@@ -2133,6 +2781,14 @@ static int fused_chunks(Context &ctx, FusedParams &P, int nslots, bool perstep)
         if (P.nt <= 0 || P.nt > ctx.fused_chunk) {
             set_error("internal: tracer chunk outside the fused workspace");
             return -1;
+        }
+        P.order = nullptr;
+        if (!perstep && !P.explicit_seg && packed_rule(ctx, P)) {
+            int *order = ctx.d_order + 2 * kOrderBins;
+            CROMA_CUDA(launch_order(ctx.stream, P.nt, P.a.sched.nsub + P.t0, reinterpret_cast<unsigned *>(ctx.d_order),
+                                    order));
+            P.order = order;
+            ctx.last_launches += P.nt <= kOrderOneBlock ? 1 : 2;
         }
         if (!cap && !perstep) {
             // one launch per kernel for the chunk: the upload wait and the

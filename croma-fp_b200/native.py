@@ -469,7 +469,7 @@ class TracerFP:
         del keep
 
     SOLVERS = {0: "thomas-scan", 1: "thomas-scan-fp32-refined", 2: "pcr", 3: "thomas-scan-smem",
-               4: "thomas-scan-rhs-smem", 5: "thomas-scan4"}
+               4: "thomas-scan-rhs-smem", 5: "thomas-scan4", 6: "thomas-scan-packed"}
     VARIANTS = ("scan x1", "scan x2", "smem scan x1", "smem scan x2", "pcr x1", "rhs scan x1", "rhs scan x2",
                 "scan4 x1", "scan4 x2")
 

@@ -316,30 +316,30 @@ typedef struct {
 } CromaB200StepHost;
 int croma_b200_step_host(CromaB200Context *ctx, const CromaB200Snapshot *snap, const CromaB200StepHost *io);
 
-/* The steps-kernel autotuner (the on-chip FP64 path).  The arithmetic is
- * fixed by rule, so that no result depends on a timing: the short-chain warp
- * scan (radix-4 warp scans, the back substitution's local pass overlapping
- * the forward scan) at 512 bins and more, the warp scan below, warp PCR (one
- * warp per tracer, parallel cyclic reduction in shared memory) when
- * CROMA_CUDA_TRIDIAG=pcr (src/fp_cuda_solver.cu:41-72 of the reference).
- * Within that family the variants compute bit-identical results and differ
- * in where the per-segment constants live -- registers, partly shared memory
- * (fewer registers, more warps per SM), or with each row's right-hand-side
- * scaling in shared memory too -- and in tracers (warps) per block, 1 or 2.
- * On the first workspace chunk a context evolves, per species, each of them
- * runs the chunk's first tracers (up to 16,384, several full waves of every
- * variant) for 16 sub-steps on a copy of their spectra, timed with CUDA
- * events, and the fastest is kept for the context; a calibration on the full
- * 16,384 tracers is reused by the process's later contexts (same species,
- * source and CROMA_CUDA_TRIDIAG).  Reported here: tuned (0 before the first
- * snapshot), solver (0 scan, 1 FP32-refined scan, 2 PCR, 3 scan with
- * shared-memory constants, 4 scan with the right-hand-side scaling in shared
- * memory, 5 short-chain scan), tracers per block, and the calibration time of
- * each variant in milliseconds, variant_ms[CROMA_B200_STEPS_VARIANTS] in the
- * order scan x1, scan x2, shared scan x1, shared scan x2, PCR, rhs-shared
- * scan x1, rhs-shared scan x2, short-chain scan x1, short-chain scan x2
- * (-1 = not run).  CROMA_B200_STEPS_VARIANT=0..8 fixes the variant in that
- * order without calibrating (reproducible profiles). */
+/* The steps kernel of the on-chip FP64 path.  The arithmetic is fixed by
+ * rule, so that no result depends on a timing: from 64 tracers on the packed
+ * scan (16 rows a lane, several tracers a warp below 512 bins; no
+ * calibration), warp PCR (one warp per tracer, parallel cyclic reduction in
+ * shared memory) when CROMA_CUDA_TRIDIAG=pcr (src/fp_cuda_solver.cu:41-72 of
+ * the reference), and for fewer tracers the short-chain warp scan (radix-4
+ * warp scans, the back substitution's local pass overlapping the forward scan)
+ * at 512 bins and more, the warp scan below.  Within those last families the
+ * variants compute bit-identical results and differ in where the per-segment
+ * constants live -- registers, partly shared memory (fewer registers, more
+ * warps per SM), or with each row's right-hand-side scaling in shared memory
+ * too -- and in tracers (warps) per block, 1 or 2.  On the first workspace
+ * chunk a context evolves, per species, each of them runs the chunk's first
+ * tracers (up to 16,384) for 16 sub-steps on a copy of their spectra, timed
+ * with CUDA events, and the fastest is kept for the context.  Reported here:
+ * tuned (0 before the first snapshot), solver (0 scan, 1 FP32-refined scan, 2
+ * PCR, 3 scan with shared-memory constants, 4 scan with the right-hand-side
+ * scaling in shared memory, 5 short-chain scan, 6 packed scan), tracers per
+ * block, and the calibration time of each variant in milliseconds,
+ * variant_ms[CROMA_B200_STEPS_VARIANTS] in the order scan x1, scan x2, shared
+ * scan x1, shared scan x2, PCR, rhs-shared scan x1, rhs-shared scan x2,
+ * short-chain scan x1, short-chain scan x2 (-1 = not run).
+ * CROMA_B200_STEPS_VARIANT=0..8 fixes the variant in that order without
+ * calibrating (reproducible profiles). */
 #define CROMA_B200_STEPS_VARIANTS 9
 int croma_b200_get_tuning(CromaB200Context *ctx, int species, int *tuned, int *solver, int *warps_per_block,
                           double *variant_ms);
