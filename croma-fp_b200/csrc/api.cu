@@ -134,7 +134,7 @@ int ic_slot(Context &c, double z, int avoid_slot, double **out)
     c.ic_valid[k] = 1;
     c.ic_z[k] = z;
     *out = c.d_ic + (size_t)k * kIcSlotDoubles;
-    c.last_launches += 1;
+    c.last_launches += 2;
     return k;
 }
 
@@ -227,6 +227,7 @@ void croma_b200_destroy(CromaB200Context *h)
     dev_free(c, c.d_tables);
     dev_free(c, c.d_np_min_qe);
     dev_free(c, c.d_ic);
+    dev_free(c, c.d_ic_work);
     dev_free(c, c.d_err);
     free_ic_stage(c);
     free_dsa(c);

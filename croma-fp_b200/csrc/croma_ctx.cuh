@@ -109,6 +109,8 @@ struct Context {
     double ic_z[2] = {0, 0};
     int ic_valid[2] = {0, 0};
     int ic_slot_curr = 0;
+    double *d_ic_work = nullptr;      // inner abscissae of the IC rows (grow-only)
+    size_t ic_work_doubles = 0;
     // pinned staging of the IC outer abscissae: two slots, each reused only
     // after the copy that last read it has completed (its event)
     double *h_ic_stage = nullptr;

@@ -261,13 +261,13 @@ constexpr double kExpInvL = 0x1.71547652b82fep+5;   // 32 / ln2
 constexpr double kExpLhi = 0x1.62e42fefa39efp-6;    // ln2 / 32, leading part
 constexpr double kExpLlo = 0x1.abc9e3b39803fp-61;   // ln2 / 32 - kExpLhi
 
-CROMA_HD double exp_tab(double x)
+#ifdef __CUDACC__
+// 2^(j/32) exp(r), j the low five bits of N: exp(x) = 2^(N >> 5) times it
+__device__ __forceinline__ double exp_tab_fraction(double x, int &N)
 {
-#ifdef __CUDA_ARCH__
-    x = x < -746.0 ? -746.0 : (x > 709.0 ? 709.0 : x);   // a NaN passes through
     const double t = fma(x, kExpInvL, 0x1.8p52);
     const double n = t - 0x1.8p52;
-    const int N = __double2loint(t);
+    N = __double2loint(t);
     double r = fma(-n, kExpLhi, x);
     r = fma(-n, kExpLlo, r);
     const double r2 = r * r;
@@ -276,13 +276,37 @@ CROMA_HD double exp_tab(double x)
     v = fma(1.0 / 720.0, r2, v);
     const double p = fma(fma(v, r2, u), r2, r);
     const double tj = __ldg(&kExp2J[N & 31]);
+    return fma(tj, p, tj);
+}
+#endif
+CROMA_HD double exp_tab(double x)
+{
+#ifdef __CUDA_ARCH__
+    x = x < -746.0 ? -746.0 : (x > 709.0 ? 709.0 : x);   // a NaN passes through
+    int N;
+    const double f = exp_tab_fraction(x, N);
     const int m = N >> 5, m1 = m >> 1, m2 = m - m1;
     const double s1 = __hiloint2double((m1 + 1023) << 20, 0), s2 = __hiloint2double((m2 + 1023) << 20, 0);
-    return fma(tj, p, tj) * s1 * s2;
+    return f * s1 * s2;
 #else
     return exp(x);
 #endif
 }
+#ifdef __CUDACC__
+// exp_tab for |x| < 708 (exp_tab_normal_range): the result is a normal number, so
+// the power of two goes straight into its exponent field -- the same value in
+// half the instructions.
+__device__ __forceinline__ bool exp_tab_normal_range(double x)   // false for a NaN
+{
+    return (__double2hiint(x) & 0x7fffffff) < 0x40862000;
+}
+__device__ __forceinline__ double exp_tab_normal(double x)
+{
+    int N;
+    const double f = exp_tab_fraction(x, N);
+    return __hiloint2double(__double2hiint(f) + ((N & ~31) << 15), __double2loint(f));
+}
+#endif
 
 // The same weights with one exponential and one division per face and no
 // divergent branch (the evolve kernels' form): exp(-w/2) is taken as
@@ -329,17 +353,6 @@ struct IcConsts {
     double log10_90;      // 90 log(10)
 };
 
-CROMA_HD double ic_kernel(double eps0, double gamma, double eps)   // IC_kernel :379-389
-{
-    const double re = 2.82e-13;
-    const double kappa = eps / (4.0 * eps0 * gamma * (gamma - eps));
-    if (kappa <= 0.0) return 0.0;
-    const double t = 4.0 * eps0 * kappa * gamma;
-    double C = 2.0 * kappa * log(kappa) + (1.0 + 2.0 * kappa) * (1.0 - kappa) +
-               (t * t) / (2.0 * (1.0 + 4.0 * eps0 * gamma * kappa)) * (1.0 - kappa);
-    return 2.0 * kPi * re * re * kC / (gamma * gamma * eps0) * C;
-}
-
 CROMA_HD double cmb_density(const IcConsts &k, double eps, double z)   // :391-406
 {
     const double Tcmb = 2.757 * (1.0 + z);
@@ -359,56 +372,6 @@ CROMA_HD double cmb_density_deps(const IcConsts &k, double eps, double z)   // :
     const double ex = exp(X);
     return k.cmb_pref_d * eps / (ex - 1.0) *
            (2.0 - eps * 9.11e-28 * kC * kC * ex / (k.k_d * Tcmb * (ex - 1.0)));
-}
-
-// Inner integral b_IC_integrand (FP_Coef.c:512-539)
-CROMA_HD double b_ic_integrand(double eps0, double gamma, double emin, double emax)
-{
-    const double da = 0.50e-1;
-    const int N = (int)round((log10(emax) - log10(emin)) / da);
-    double a = log10(emin), epsnew = emin, integral = 0.0;
-    double newC = ic_kernel(eps0, gamma, epsnew);
-    for (int i = 0; i < N; i++) {
-        a = a + da;
-        const double eps = epsnew;
-        epsnew = pow(10.0, a);
-        const double deps = epsnew - eps;
-        const double C = newC;
-        newC = ic_kernel(eps0, gamma, epsnew);
-        integral = integral + 0.5 * (eps * C + epsnew * newC) * deps;
-    }
-    return integral;
-}
-
-// IC_emissivity_kernel, FP_Coef.c:553-584: the inverse-Compton emissivity of
-// one electron of Lorentz factor gamma at frequency nu (Hz), a 400-step
-// log-spaced trapezoid over the seed CMB photon energy.  The photon energy
-// is normalised with the routine's own c = 3.0e10.
-CROMA_HD double ic_emissivity(const IcConsts &k, double nu, double gamma, double z)
-{
-    const int N = 400;
-    const double meg = 9.11e-28, c_local = 3.0e+10;
-    const double eps = kHPlanck * nu / (meg * c_local * c_local);
-    const double e0max = eps;
-    double e0min = eps / (4.0 * gamma * (gamma - eps));
-    if (e0min < 0) e0min = eps / (gamma * gamma);
-    const double da = (log10(e0max) - log10(e0min)) / (double)N;
-    double a = log10(e0min);
-    double eps0new = pow(10.0, a);
-    double Cnew = ic_kernel(eps0new, gamma, eps);
-    double n0new = cmb_density(k, eps0new, z);
-    double integral = 0.0;
-    for (int i = 0; i < N; i++) {
-        a = a + da;
-        const double eps0 = eps0new;
-        eps0new = pow(10.0, a);
-        const double deps0 = eps0new - eps0;
-        const double C = Cnew, n = n0new;
-        n0new = cmb_density(k, eps0new, z);
-        Cnew = ic_kernel(eps0new, gamma, eps);
-        integral = integral + 0.5 * (C * n + Cnew * n0new) * deps0;
-    }
-    return kHPlanck * eps * integral / (4.0 * kPi);
 }
 
 }  // namespace croma

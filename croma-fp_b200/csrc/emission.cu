@@ -112,12 +112,62 @@ __global__ void neutrino_table_kernel(int nbins, const double *E, const double *
     out[i] = neutrino_kernel(E[i / NB], p[i % NB]);
 }
 
-__global__ void ic_table_kernel(IcConsts k, int nbins, const double *nu, const double *p, double z, double *out)
+// IC_emissivity_kernel, FP_Coef.c:553-584: the inverse-Compton emissivity of
+// one electron of Lorentz factor gamma at frequency nu (Hz), a 400-step
+// log-spaced trapezoid over the seed CMB photon energy eps0, a warp per (band,
+// momentum bin) with its lanes along the steps.  The photon energy is
+// normalised with the routine's own c = 3.0e10.  IC_kernel (FP_Coef.c:379-389)
+// with t = eps / (gamma - eps) = 4 eps0 kappa gamma, which the steps share:
+// kappa = t / (4 gamma eps0), and a factor 2 pi r_e^2 c / gamma^2 taken out.
+// A thread per entry walked the 400 steps, a power, a logarithm, an exponential
+// and four divisions each, with 1,024 warps on the chip: 407 us per snapshot
+// at 64 bands x 512 bins; now 87 us.
+__global__ void __launch_bounds__(256) ic_table_kernel(IcConsts k, int nbins, const double *nu, const double *p, double z,
+                                                       double *out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= nbins * NB) return;
-    const double pe = p[i % NB];
-    out[i] = ic_emissivity(k, nu[i / NB], sqrt(1.0 + pe * pe), z);
+    constexpr int N = 400;
+    constexpr double meg = 9.11e-28, c_local = 3.0e+10, re = 2.82e-13;
+    const double pe = p[i % NB], gamma = sqrt(1.0 + pe * pe);
+    const double eps = kHPlanck * nu[i / NB] / (meg * c_local * c_local);
+    double e0min = eps / (4.0 * gamma * (gamma - eps));
+    if (e0min < 0) e0min = eps / (gamma * gamma);
+    const double a0 = log10(e0min), da = (log10(eps) - a0) / (double)N;
+    const double t = eps / (gamma - eps), k4 = t / (4.0 * gamma), t2 = t * t / (2.0 * (1.0 + t));
+    const double Tcmb = 2.757 * (1.0 + z), xk = 9.11e-28 * kC * kC / (1.38e-16 * Tcmb);
+    double sum = 0.0, f_last = 0.0, e_last = 0.0;
+    for (int base = 0; base <= N; base += 32) {
+        const int s = base + lane;
+        double e = 0.0, f = 0.0;
+        if (s <= N) {
+            e = exp10(fma((double)s, da, a0));
+            const double ie = rcp_nr(e), kappa = k4 * ie;
+            if (!(kappa <= 0.0)) {
+                const double C = 2.0 * kappa * log(kappa) + (1.0 + 2.0 * kappa) * (1.0 - kappa) + t2 * (1.0 - kappa);
+                // cmb_density, FP_Coef.c:391-406
+                const double X = e * xk;
+                double n = 0.0;
+                if (!(X > k.log10_90)) {
+                    const double ex = exp(X) - 1.0;
+                    n = ex < 1.0e-40 ? k.cmb_pref * e / (9.11e-28 * kC * kC * (1.0 + 0.5 * X + X / 6.0) / (1.38e-16 * Tcmb))
+                                     : k.cmb_pref * (e * e) * rcp_nr(ex);
+                }
+                f = C * ie * n;
+            }
+        }
+        double fp = __shfl_up_sync(kFull, f, 1), ep = __shfl_up_sync(kFull, e, 1);
+        if (lane == 0) {
+            fp = f_last;
+            ep = e_last;
+        }
+        if (s >= 1 && s <= N) sum += 0.5 * (fp + f) * (e - ep);
+        f_last = __shfl_sync(kFull, f, 31);
+        e_last = __shfl_sync(kFull, e, 31);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
+    if (lane == 0) out[i] = kHPlanck * eps * (sum * (2.0 * kPi * re * re * kC / (gamma * gamma))) / (4.0 * kPi);
 }
 
 // logy[nf][je][k] = log10(nu_nf / (1e-6 nu_crit[je][k])), nu_crit the
@@ -151,18 +201,33 @@ __global__ void log_table_kernel(long long n, const double *K, double *logK)
 }
 
 // ---------------------------------------------------------------------------
-// Emissivity GEMM: out[t][k] = scale[t] * sum_j N[t][j] W[j][k] for k < ncols,
-// N the resident spectra [ntracer][NB], W [NB][wpitch] (zero past ncols).
-// FP64 tensor cores (mma.sync m8n8k4 .f64); 128 x 64 output tile per 256
-// threads, each warp 32 x 32 as 4 x 4 fragments; k-tiles of 16 double-buffered
-// in shared memory by cp.async.  Row pitches 20 and 68 doubles keep the
-// fragment reads of a half warp on distinct bank pairs.
-constexpr int kEM = 128, kEN = 64, kEK = 16;
+// Emissivity GEMMs: out[t][k] = scale[t] * sum_j N[t][j] W[j][k] for k < ncols,
+// N the resident spectra [ntracer][NB], W [NB][wpitch] (zero past ncols), of up
+// to three kinds (IC, gamma, neutrino) in one launch.  FP64 tensor cores
+// (mma.sync m8n8k4 .f64); MT x 64 output tile per 256 threads; k-tiles of 16
+// double-buffered in shared memory by cp.async.  Row pitches 20 and 68 doubles
+// keep the fragment reads of a half warp on distinct bank pairs.
+// A tile of 128 rows (each warp 32 x 32) keeps an SM's FP64 tensor pipe busy for
+// 33 us; where such tiles do not fill the chip, tiles of 32 rows (16 x 16 a
+// warp) take a quarter of that each.  1,500 tracers, 512 bins, 3 x 64 bands: three
+// launches of 12 blocks 138 us, now 20 us; 131,072 tracers 834 us, now 809 us.
+constexpr int kEN = 64, kEK = 16;
 constexpr int kEPitchA = kEK + 4, kEPitchB = kEN + 4;
 
+template <int MT>
 struct EmisGemmSmem {
-    double A[2][kEM][kEPitchA];
+    double A[2][MT][kEPitchA];
     double B[2][kEK][kEPitchB];
+};
+
+struct EmisKind {
+    int ncols, wpitch, first;   // first: this kind's first column tile in the launch
+    const double *N, *W, *scale;
+    double *out;
+};
+struct EmisGemm {
+    int nrows, nkinds, ntiles;  // ntiles: column tiles of all kinds
+    EmisKind k[3];
 };
 
 __device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
@@ -179,42 +244,47 @@ __device__ __forceinline__ void mma_f64(double &d0, double &d1, double a, double
                  : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(256, 2) emission_gemm_kernel(int nrows, int ncols, int wpitch, const double *N,
-                                                               const double *W, const double *scale,
-                                                               int scale_stride, double *out)
+template <int MT>
+__global__ void __launch_bounds__(256, 2) emission_gemm_kernel(EmisGemm G)
 {
+    constexpr int F = MT == 128 ? 4 : 2;             // fragments of a warp's tile, each way
+    constexpr int WN = kEN / (8 * F);                // warps along the columns
     extern __shared__ double4 smem_raw[];
-    EmisGemmSmem &sm = *reinterpret_cast<EmisGemmSmem *>(smem_raw);
+    EmisGemmSmem<MT> &sm = *reinterpret_cast<EmisGemmSmem<MT> *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = (warp / WN) * (8 * F), wn = (warp % WN) * (8 * F);
     const int gid = lane >> 2, tig = lane & 3;
-    const int ntile_n = wpitch / kEN;
-    const int n0 = (int)(blockIdx.x % ntile_n) * kEN;
-    const long long m0 = (long long)(blockIdx.x / ntile_n) * kEM;
+    const int tile = (int)(blockIdx.x % G.ntiles);
+    const long long m0 = (long long)(blockIdx.x / G.ntiles) * MT;
+    int kind = 0;
+    if (G.nkinds > 1 && tile >= G.k[1].first) kind = 1;
+    if (G.nkinds > 2 && tile >= G.k[2].first) kind = 2;
+    const EmisKind K = G.k[kind];
+    const int n0 = (tile - K.first) * kEN, nrows = G.nrows;
 
     auto load_tile = [&](int buf, int k0) {
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < MT / 32; c++) {
             const int q = tid + 256 * c;   // row q / 8, 16-byte chunk q % 8
             const int r = q >> 3, ch = q & 7;
             const long long m = m0 + r;
             const bool ok = m < nrows;
-            cp16(&sm.A[buf][r][ch * 2], N + (size_t)(ok ? m : 0) * NB + k0 + ch * 2, ok);
+            cp16(&sm.A[buf][r][ch * 2], K.N + (size_t)(ok ? m : 0) * NB + k0 + ch * 2, ok);
         }
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const int q = tid + 256 * c;   // row q / 32, chunk q % 32
             const int r = q >> 5, ch = q & 31;
-            cp16(&sm.B[buf][r][ch * 2], W + (size_t)(k0 + r) * wpitch + n0 + ch * 2, true);
+            cp16(&sm.B[buf][r][ch * 2], K.W + (size_t)(k0 + r) * K.wpitch + n0 + ch * 2, true);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    double acc[4][4][2];
+    double acc[F][F][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < F; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < F; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
     load_tile(0, 0);
     int buf = 0;
@@ -229,30 +299,30 @@ __global__ void __launch_bounds__(256, 2) emission_gemm_kernel(int nrows, int nc
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < kEK; kk += 4) {
-            double af[4], bf[4];
+            double af[F], bf[F];
 #pragma unroll
-            for (int i = 0; i < 4; i++) af[i] = sm.A[buf][wm + 8 * i + gid][kk + tig];
+            for (int i = 0; i < F; i++) af[i] = sm.A[buf][wm + 8 * i + gid][kk + tig];
 #pragma unroll
-            for (int j = 0; j < 4; j++) bf[j] = sm.B[buf][kk + tig][wn + 8 * j + gid];
+            for (int j = 0; j < F; j++) bf[j] = sm.B[buf][kk + tig][wn + 8 * j + gid];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < F; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) mma_f64(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                for (int j = 0; j < F; j++) mma_f64(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
         }
         __syncthreads();
         buf ^= 1;
     }
     // fragment (i, j): C[wm + 8i + gid][wn + 8j + 2 tig + {0, 1}]
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < F; i++) {
         const long long m = m0 + wm + 8 * i + gid;
         if (m >= nrows) continue;
-        const double s = scale ? scale[(size_t)m * scale_stride] : 1.0;
+        const double s = K.scale ? K.scale[m] : 1.0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < F; j++) {
             const int k = n0 + wn + 8 * j + 2 * tig;
-            if (k < ncols) out[(size_t)m * ncols + k] = acc[i][j][0] * s;
-            if (k + 1 < ncols) out[(size_t)m * ncols + k + 1] = acc[i][j][1] * s;
+            if (k < K.ncols) K.out[(size_t)m * K.ncols + k] = acc[i][j][0] * s;
+            if (k + 1 < K.ncols) K.out[(size_t)m * K.ncols + k + 1] = acc[i][j][1] * s;
         }
     }
 }
@@ -282,13 +352,20 @@ __global__ void fold_weights_kernel(int nbins, int wpitch, const double *kern, c
 // The synchrotron emission with the table rows shared: tracers are sorted by
 // their lower log-B plane ib (synch_plane_kernel + a radix sort), and a block
 // of kSynWarps warps takes kSynWarps consecutive sorted tracers, one per
-// warp.  For each frequency the block stages the rows K and log K of the
-// planes its tracers interpolate between -- two or three planes when their
-// ib values span at most two, which the sort makes the common case -- in
-// shared memory, so each row is read once per block instead of once per
-// tracer.  A block whose tracers span more planes reads the table directly.
+// warp, and a range of the frequencies (blockIdx.y).  For each frequency the
+// block stages the rows log K of the planes its tracers interpolate
+// between -- two or three planes when their ib values span at most two, which
+// the sort makes the common case -- in shared memory, one frequency ahead, so
+// each row is read once per block instead of once per tracer.  A block whose
+// tracers span more planes reads the table directly.
 // Per tracer: K = exp((1 - t) log K_ib + t log K_ib+1) where both ends are
 // positive, the linear blend otherwise, clamped ends at t = 0 and 1.
+// Bound by the exponentials' instructions: they run as exp_tab_normal, four
+// rows of a lane at a time, where all of a warp's blends are in its range
+// (131,072 tracers, 64 frequencies, 512 bins: 10.4 ms with the general exp, a
+// row at a time behind its branches; now 7.7 ms).  A run whose tracers alone
+// do not fill the chip splits the frequencies over more blocks: 1,500 tracers
+// (188 blocks) 978 us, now 136 us.
 constexpr int kSynWarps = 8;
 
 __device__ __forceinline__ void synch_plane(double bval_in, double logb_min, double inv_dlogb, int nlogb, int &ib,
@@ -319,10 +396,10 @@ __global__ void synch_plane_kernel(int ntracer, int nlogb, double logb_min, doub
 }
 
 struct SynRows {
-    double K[3][NB], L[3][NB];
+    double L[2][3][NB];   // log K of the block's planes at this frequency and the next
 };
 
-__global__ void __launch_bounds__(kSynWarps * 32, 3) synch_sorted_kernel(
+__global__ void __launch_bounds__(kSynWarps * 32, 2) synch_sorted_kernel(
     int ntracer, int nfreq, int nlogb, double logb_min, double inv_dlogb, SynchPrefactor sp, const double *K,
     const double *logK, const int *order, const double *bfield, const double *cre, const double *dp, double *out)
 {
@@ -341,6 +418,15 @@ __global__ void __launch_bounds__(kSynWarps * 32, 3) synch_sorted_kernel(
     synch_plane(bfield[order[last]], logb_min, inv_dlogb, nlogb, ib_hi, tw_unused);
     const bool staged = ib_hi - ib_lo <= 1;
     const int nplanes = staged ? ib_hi - ib_lo + 2 : 0;
+    const int f0 = (int)((long long)nfreq * blockIdx.y / gridDim.y);
+    const int f1 = (int)((long long)nfreq * (blockIdx.y + 1) / gridDim.y);
+    auto stage = [&](int nf, int buf) {
+        for (int i = threadIdx.x; i < nplanes * (NB / 2); i += blockDim.x) {
+            const int pl = i / (NB / 2), c = i % (NB / 2);
+            cp16(&rows.L[buf][pl][2 * c], logK + ((size_t)(ib_lo + pl) * nfreq + nf) * NB + 2 * c, true);
+        }
+    };
+    if (staged && f0 < f1) stage(f0, 0);
     const int t = active ? order[pos] : 0;
     const double *N = cre + (size_t)t * NB;
     int stop = NB - 1;
@@ -363,41 +449,50 @@ __global__ void __launch_bounds__(kSynWarps * 32, 3) synch_sorted_kernel(
     synch_plane(active ? bfield[t] : 1.0, logb_min, inv_dlogb, nlogb, ib, tw);
     const double A = active ? sp.a0 * bfield[t] / sp.den1 / sp.den2 : 0.0;
     const int s0 = ib - ib_lo;   // staged row of plane ib
-    for (int nf = 0; nf < nfreq; nf++) {
+    for (int nf = f0; nf < f1; nf++) {
+        const int buf = (nf - f0) & 1;
         if (staged) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < nplanes * NB; i += blockDim.x) {
-                const int pl = i / NB, je = i % NB;
-                const size_t o = ((size_t)(ib_lo + pl) * nfreq + nf) * NB + je;
-                rows.K[pl][je] = __ldg(K + o);
-                rows.L[pl][je] = __ldg(logK + o);
-            }
-            __syncthreads();
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();   // this frequency's rows are in, the other buffer's are read
+            if (nf + 1 < f1) stage(nf + 1, buf ^ 1);
         }
         if (!active) continue;
         const size_t o0 = ((size_t)ib * nfreq + nf) * NB, o1 = ((size_t)(ib + 1) * nfreq + nf) * NB;
         double sum = 0.0;
+        if (tw <= 0.0 || tw >= 1.0) {
+            const double *Krow = K + (tw <= 0.0 ? o0 : o1);
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int je = 32 * r + lane;
-            if (nd[r] == 0.0) continue;
-            double Kv;
-            if (tw <= 0.0) {
-                Kv = staged ? rows.K[s0][je] : __ldg(K + o0 + je);
-            } else if (tw >= 1.0) {
-                Kv = staged ? rows.K[s0 + 1][je] : __ldg(K + o1 + je);
-            } else {
-                const double la = staged ? rows.L[s0][je] : __ldg(logK + o0 + je);
-                const double lb = staged ? rows.L[s0 + 1][je] : __ldg(logK + o1 + je);
-                if (!isnan(la) && !isnan(lb)) {
-                    Kv = exp((1.0 - tw) * la + tw * lb);
-                } else {
-                    const double ka = staged ? rows.K[s0][je] : __ldg(K + o0 + je);
-                    const double kb = staged ? rows.K[s0 + 1][je] : __ldg(K + o1 + je);
-                    Kv = (1.0 - tw) * ka + tw * kb;
+            for (int r = 0; r < R; r++)
+                if (nd[r] != 0.0) sum += nd[r] * __ldg(Krow + 32 * r + lane);
+        } else {
+            const double *La = staged ? rows.L[buf][s0] : logK + o0, *Lb = staged ? rows.L[buf][s0 + 1] : logK + o1;
+#pragma unroll
+            for (int r = 0; r < R; r += 4) {
+                double x[4];
+                bool plain = true;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int je = 32 * (r + i) + lane;
+                    x[i] = (1.0 - tw) * La[je] + tw * Lb[je];   // NaN where an end is not positive
+                    plain &= exp_tab_normal_range(x[i]);
+                }
+                if (__all_sync(kFull, plain)) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) sum += nd[r + i] * exp_tab_normal(x[i]);
+                    continue;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    double e = 0.0;   // both ends zero (a NaN spectrum stays one)
+                    if (!isnan(x[i])) {
+                        e = exp_tab(x[i]);
+                    } else if (isnan(La[32 * (r + i) + lane]) != isnan(Lb[32 * (r + i) + lane])) {
+                        const int je = 32 * (r + i) + lane;
+                        e = (1.0 - tw) * __ldg(K + o0 + je) + tw * __ldg(K + o1 + je);
+                    }
+                    sum += nd[r + i] * e;
                 }
             }
-            sum += nd[r] * Kv;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
@@ -469,7 +564,7 @@ cudaError_t launch_table(int kind, int nbins, const double *d_E, const double *d
     const int blocks = (n + 127) / 128;
     if (kind == kTabGamma) gamma_table_kernel<<<blocks, 128, 0, st>>>(nbins, d_E, d_p, d_out);
     else if (kind == kTabNeutrino) neutrino_table_kernel<<<blocks, 128, 0, st>>>(nbins, d_E, d_p, d_out);
-    else ic_table_kernel<<<blocks, 128, 0, st>>>(ic_consts(), nbins, d_E, d_p, z, d_out);
+    else ic_table_kernel<<<(n + 7) / 8, 256, 0, st>>>(ic_consts(), nbins, d_E, d_p, z, d_out);
     return cudaGetLastError();
 }
 
@@ -543,17 +638,40 @@ namespace {
 
 int pad64(int n) { return (n + 63) / 64 * 64; }
 
-cudaError_t launch_gemm(int nrows, int ncols, int wpitch, const double *N, const double *W, const double *scale,
-                        int scale_stride, double *out, cudaStream_t st)
+int sm_count()
 {
-    constexpr size_t smem = sizeof(EmisGemmSmem);
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
+template <int MT>
+cudaError_t launch_gemm_tile(const EmisGemm &G, cudaStream_t st)
+{
+    constexpr size_t smem = sizeof(EmisGemmSmem<MT>);
     static const cudaError_t attr =
-        cudaFuncSetAttribute(emission_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(emission_gemm_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess) return attr;
-    const long long blocks = ((long long)nrows + kEM - 1) / kEM * (wpitch / kEN);
+    const long long blocks = ((long long)G.nrows + MT - 1) / MT * G.ntiles;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    emission_gemm_kernel<<<(unsigned)blocks, 256, smem, st>>>(nrows, ncols, wpitch, N, W, scale, scale_stride, out);
+    emission_gemm_kernel<MT><<<(unsigned)blocks, 256, smem, st>>>(G);
     return cudaGetLastError();
+}
+
+void add_kind(EmisGemm &G, int ncols, int wpitch, const double *N, const double *W, const double *scale, double *out)
+{
+    G.k[G.nkinds++] = EmisKind{ncols, wpitch, G.ntiles, N, W, scale, out};
+    G.ntiles += wpitch / kEN;
+}
+
+// Tiles of 128 rows once they give every SM two blocks (what it holds); the
+// sums are the same either way.
+cudaError_t launch_gemm(const EmisGemm &G, cudaStream_t st)
+{
+    if (G.nkinds == 0) return cudaSuccess;
+    const long long big = ((long long)G.nrows + 127) / 128 * G.ntiles;
+    return big >= 2LL * sm_count() ? launch_gemm_tile<128>(G, st) : launch_gemm_tile<32>(G, st);
 }
 
 int setup_emission(Context &c, const CromaB200EmissionSetup *s)
@@ -717,6 +835,8 @@ int emission_run(Context &c, const double *bg, double z, double *eps_syn, double
     const int n = c.ntracer;
     cudaStream_t st = c.stream;
     e->ic_rebuilt = 0;
+    EmisGemm gemm{};
+    gemm.nrows = n;
     if (eps_ic && s.nbins_ic > 0) {
         if (!e->ic_valid || e->ic_z != z) {
             e->ic_rebuilt = 1;
@@ -728,13 +848,12 @@ int emission_run(Context &c, const double *bg, double z, double *eps_syn, double
             e->ic_z = z;
             e->ic_valid = 1;
         }
-        CROMA_CUDA(launch_gemm(n, s.nbins_ic, e->wp_ic, c.d_cre, e->d_w_ic, nullptr, 0, eps_ic, st));
+        add_kind(gemm, s.nbins_ic, e->wp_ic, c.d_cre, e->d_w_ic, nullptr, eps_ic);
     }
     // n_gas is field 0 of the field-major background [8][ntracer]
-    if (eps_gamma && s.nbins_gamma > 0)
-        CROMA_CUDA(launch_gemm(n, s.nbins_gamma, e->wp_gamma, c.d_crp, e->d_w_gamma, bg, 1, eps_gamma, st));
-    if (eps_nu && s.nbins_nu > 0)
-        CROMA_CUDA(launch_gemm(n, s.nbins_nu, e->wp_nu, c.d_crp, e->d_w_nu, bg, 1, eps_nu, st));
+    if (eps_gamma && s.nbins_gamma > 0) add_kind(gemm, s.nbins_gamma, e->wp_gamma, c.d_crp, e->d_w_gamma, bg, eps_gamma);
+    if (eps_nu && s.nbins_nu > 0) add_kind(gemm, s.nbins_nu, e->wp_nu, c.d_crp, e->d_w_nu, bg, eps_nu);
+    CROMA_CUDA(launch_gemm(gemm, st));
     if (eps_syn && s.nfreq > 0) {
         const double *bfield = bg + 2 * (size_t)n;
         if (e->sort_cap < n) {
@@ -766,7 +885,12 @@ int emission_run(Context &c, const double *bg, double z, double *eps_syn, double
         static const cudaError_t attr =
             cudaFuncSetAttribute(synch_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         CROMA_CUDA(attr);
-        synch_sorted_kernel<<<(n + kSynWarps - 1) / kSynWarps, kSynWarps * 32, smem, st>>>(
+        // frequencies split over blocks until the chip (2 blocks an SM) is filled
+        // twice; each block's own cost, its spectra, is that of one frequency
+        const long long blocks = ((long long)n + kSynWarps - 1) / kSynWarps;
+        const long long want = 4LL * sm_count() / blocks;
+        const unsigned split = (unsigned)(want < 1 ? 1 : (want > s.nfreq ? s.nfreq : want));
+        synch_sorted_kernel<<<dim3((unsigned)blocks, split), kSynWarps * 32, smem, st>>>(
             n, s.nfreq, s.nlogb, s.logb_min, e->inv_dlogb, synch_prefactor(), e->d_K, e->d_logK, vb.Current(),
             bfield, c.d_cre, c.gt.s[1].dp, eps_syn);
         CROMA_CUDA(cudaGetLastError());
@@ -798,8 +922,8 @@ int emission_launches(const Context &c, bool syn, bool ic, bool gamma, bool nu)
 {
     const EmissionState *e = c.emission;
     if (!e) return 0;
-    return 3 * (syn && e->cfg.nfreq > 0) + (ic && e->cfg.nbins_ic > 0) * (1 + 2 * e->ic_rebuilt) +
-           (gamma && e->cfg.nbins_gamma > 0) + (nu && e->cfg.nbins_nu > 0);
+    const bool any = (ic && e->cfg.nbins_ic > 0) || (gamma && e->cfg.nbins_gamma > 0) || (nu && e->cfg.nbins_nu > 0);
+    return 3 * (syn && e->cfg.nfreq > 0) + (ic && e->cfg.nbins_ic > 0) * 2 * e->ic_rebuilt + any;
 }
 
 int emission_tables(Context &c, int which, double *out)
