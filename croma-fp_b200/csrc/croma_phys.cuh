@@ -263,7 +263,8 @@ constexpr double kExpLlo = 0x1.abc9e3b39803fp-61;   // ln2 / 32 - kExpLhi
 
 #ifdef __CUDACC__
 // 2^(j/32) exp(r), j the low five bits of N: exp(x) = 2^(N >> 5) times it
-__device__ __forceinline__ double exp_tab_fraction(double x, int &N)
+template <class Entry>
+__device__ __forceinline__ double exp_tab_fraction(double x, int &N, Entry entry)
 {
     const double t = fma(x, kExpInvL, 0x1.8p52);
     const double n = t - 0x1.8p52;
@@ -275,7 +276,7 @@ __device__ __forceinline__ double exp_tab_fraction(double x, int &N)
     double v = fma(1.0 / 120.0, r, 1.0 / 24.0);
     v = fma(1.0 / 720.0, r2, v);
     const double p = fma(fma(v, r2, u), r2, r);
-    const double tj = __ldg(&kExp2J[N & 31]);
+    const double tj = entry(N & 31);   // 2^(j/32)
     return fma(tj, p, tj);
 }
 #endif
@@ -284,7 +285,7 @@ CROMA_HD double exp_tab(double x)
 #ifdef __CUDA_ARCH__
     x = x < -746.0 ? -746.0 : (x > 709.0 ? 709.0 : x);   // a NaN passes through
     int N;
-    const double f = exp_tab_fraction(x, N);
+    const double f = exp_tab_fraction(x, N, [](int j) { return __ldg(&kExp2J[j]); });
     const int m = N >> 5, m1 = m >> 1, m2 = m - m1;
     const double s1 = __hiloint2double((m1 + 1023) << 20, 0), s2 = __hiloint2double((m2 + 1023) << 20, 0);
     return f * s1 * s2;
@@ -300,11 +301,16 @@ __device__ __forceinline__ bool exp_tab_normal_range(double x)   // false for a 
 {
     return (__double2hiint(x) & 0x7fffffff) < 0x40862000;
 }
-__device__ __forceinline__ double exp_tab_normal(double x)
+template <class Entry>
+__device__ __forceinline__ double exp_tab_normal(double x, Entry entry)
 {
     int N;
-    const double f = exp_tab_fraction(x, N);
+    const double f = exp_tab_fraction(x, N, entry);
     return __hiloint2double(__double2hiint(f) + ((N & ~31) << 15), __double2loint(f));
+}
+__device__ __forceinline__ double exp_tab_normal(double x)
+{
+    return exp_tab_normal(x, [](int j) { return __ldg(&kExp2J[j]); });
 }
 #endif
 

@@ -6,18 +6,12 @@
 //   0. seg_pre_kernel, one thread per (segment, tracer): the segment's
 //      interpolated background and the scalars of its coefficients, once for
 //      both species.
-//   1. factor_kernel, persistent: each warp takes tracers from an atomic
-//      counter and factors every (segment[, on/off set]) of each: the loss /
-//      diffusion terms of every bin in lane-strided loops into the warp's
-//      slice of shared memory, the Chang-Cooper face weights (at 512 bins in
-//      registers, where the rows use them; below, lane-strided into shared
-//      memory) (losses / Dpp / CC assembly of src/fp_shared_core.c:729-842,
-//      1241-1317, 2358-2431 and src/Chang_Cooper.c:22-184); rows a, b, c in
-//      registers -- lane l owns rows [l*R, (l+1)*R), R = nb/32 -- and the
-//      Thomas pivots d_i = b_i - a_i c_{i-1}/d_{i-1}, a chain of Moebius maps
-//      composed per lane as 2x2 matrices and combined by a warp scan, after
-//      which each lane re-runs the exact recurrence on its rows from the
-//      scanned incoming pivot.  It stores 1/d, a/d and c/d per row.
+//   1. factor_kernel, persistent: the loss / diffusion terms, Chang-Cooper faces
+//      and rows of every (tracer, segment[, on/off set]) (losses / Dpp / CC
+//      assembly of src/fp_shared_core.c:729-842, 1241-1317, 2358-2431 and
+//      src/Chang_Cooper.c:22-184), 16 rows a lane, and the Thomas pivots d_i =
+//      b_i - a_i c_{i-1}/d_{i-1} as ratios of continuants, combined across the
+//      lanes by a scan of 2x2 matrices.  It stores 1/d, a/d and c/d per row.
 //      Nothing here depends on the evolving spectra (the eta cap aside, which
 //      then runs the chunk one segment at a time), so every segment of the
 //      snapshot is factored by one launch with full occupancy.
@@ -37,8 +31,6 @@
 //      [nb x nb] product on the FP64 tensor cores, between the proton and
 //      the electron steps.
 //
-// Shared-memory rows are stored at (m % R) * kPitch + m / R, so the blocked reads
-// of step 1 (lane l, row l*R + r and its neighbours) hit 32 distinct banks.
 // Divisions by grid quantities use reciprocals tabulated on the host; the
 // results agree with the reference's divisions to an ulp per operation.
 // Spectra are cell-major [tracer][nb] so that a warp's rows are contiguous.
@@ -53,35 +45,20 @@ namespace croma {
 namespace {
 
 constexpr int kR = NB / 32;          // rows per lane
-// Row pitch of the swizzled arrays: both access patterns of the factor
-// kernel -- lane-strided (m = 32 k + lane) and lane-blocked (m = R lane + r)
-// -- then touch 16 distinct 8-byte bank pairs per half warp.
+// Row pitch of the swizzled arrays of the PCR sub-step: lane-blocked reads (m =
+// R lane + r) and those at a stride then touch distinct bank pairs.
 constexpr int kPitch = 32 + 16 / kR;
 constexpr int kSw = kPitch * kR;     // swizzled row-array length
 // One warp per block in the steps kernels: a finished tracer's slot is
 // refilled at once instead of when the slowest warp of its block ends.
 constexpr int kWarps = 1;            // warps per block
 constexpr unsigned kFull = 0xffffffffu;
+// Packed layout (factor and packed steps kernels): 16 rows a lane at every bin
+// count, so 8, 16 or 32 lanes hold a system and a warp 4, 2 or 1 of them.
+constexpr int kPkRows = 16;
+constexpr int kPkLanes = NB / kPkRows;
+constexpr int kPkTracers = 32 / kPkLanes;
 constexpr int kFacDoubles = 3 * NB;  // 1/d, a/d, c/d of one system
-// Face weights of the factor kernel: at nb = 512 computed in registers where
-// the rows use them, so each warp's shared memory holds only B and C and one
-// 12-warp block (at most 168 registers, 160 KB of shared memory) fills an SM
-// instead of 9 warps; at nb <= 256, where registers and not shared memory
-// bound the warps, computed lane-strided into shared memory (two 9-warp
-// blocks per SM).
-constexpr bool kFacesInRegs = (NB >= 512);
-constexpr int kFacWarps = (NB <= 256 ? 9 : 12);
-
-// Grid tables of one species staged in shared memory by the factor kernel.
-// X0..X3: protons expE, cp_Ep, cp_inv2mpkin, cp_inv_betap2; electrons
-// ce_inv_beta2, ce_logp and the shared IC rows of z_curr, z_next.  RF: the
-// face factor dx / (g_j + g_j+1) of the filled Dpp form.
-enum { TB_P, TB_P2, TB_CUT, TB_2P, TB_DXF, TB_RF, TB_X0, TB_X1, TB_X2, TB_X3,
-       TB_X4,                      // protons sig_eff, in swizzled order (row loss term)
-       TB_IDX, TB_IDXL, TB_IDXR,   // 1/dp, 1/(p[m]-p[m-1]), 1/(p[m+1]-p[m]) in swizzled order
-       kTab };
-constexpr int kTabStride = (NB > kSw ? NB : kSw);   // doubles per staged table
-
 // Per-segment scalars of one (segment slot, tracer): what the factor kernels
 // of both species need of the schedule's segment and of the background
 // interpolated to it, computed once by seg_pre_kernel.
@@ -110,7 +87,6 @@ struct FusedParams {
     const double *eta_scale; // [ntracer] Dpp eta-cap scale of slot g0, or null (no cap)
     double *fac;             // [2 species][g1 - g0][sets][nt][3][nb]
     SegPre *pre;             // [g1 - g0][nt]
-    unsigned *work;          // [2] next-tracer counters of the factor kernels (per species)
     double *np_seg;          // [g1 - g0][nt][nb] proton spectra at segment starts, or null
     double *inje;            // [g1 - g0][nt][nb] electron source per segment, or null
     const int *np_min_qe;    // [nb]
@@ -179,17 +155,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-// Exact power-of-two rescaling of a 2x2 matrix (projective maps are
-// unchanged by a common factor).
-__device__ __forceinline__ void rescale2(double &m00, double &m01, double &m10, double &m11)
-{
-    const double mx = fmax(fmax(fabs(m00), fabs(m01)), fmax(fabs(m10), fabs(m11)));
-    const long long ex = (__double_as_longlong(mx) >> 52) & 0x7ff;
-    if (ex <= 0 || ex >= 2046) return;
-    const double sc = __longlong_as_double((2046LL - ex) << 52);
-    m00 *= sc; m01 *= sc; m10 *= sc; m11 *= sc;
-}
-
 // coulomb_kernel_fast with its erf / exp branch out of line: the proton
 // terms otherwise inline four copies of it, and the factor kernel's code
 // outgrows the instruction cache.  Same arithmetic.
@@ -202,77 +167,19 @@ __device__ __forceinline__ double coulomb_one(double x)
     return (x > 40.0) ? 0.5 * sqrt(kPi) : coulomb_slow(x);
 }
 
-// Per-tracer constants of species S for one segment.
-template <int S>
+// The scalars of one segment's coefficients (seg_pre_kernel).
 struct SegTerms {
-    const GridTables *gt;
     double n_gas, kbt, inv_kbt, log_n, adiab;
     double synch_coeff, coulomb_coeff;
     double dt, dt_over_tloss_pref;   // protons: dt / T = sig_eff * dt_over_tloss_pref
     double dtT_e;                    // electrons: dt / 1e100
-    double dpp_inv, dpp_scale;
-    int dpp_fill;
-    const double *ric, *ric_next;   // already offset to this tracer
-    int ric_stride;                 // bin stride of the IC row; 0: the shared row, staged
     double alpha;
     int interp;
-
-    // B = radp - 2 Dpp / p and C = Dpp at bin j, from the grid tables staged
-    // in shared memory (tab, kTab arrays of nb)
-    __device__ __forceinline__ void at(const double *tab, int j, double &B, double &C) const
-    {
-        const double p = tab[TB_P * kTabStride + j];
-        const double p2 = tab[TB_P2 * kTabStride + j];
-        const double cut = tab[TB_CUT * kTabStride + j];
-        double D;
-        if (!dpp_fill) D = p2 * (1.0 / (4.0 * 1.0e+5));
-        else if (S == 0) D = p2 * dpp_inv * tab[TB_X0 * kTabStride + j] * cut;
-        else D = p2 * dpp_inv * cut;
-        D *= dpp_scale;
-        double radp;
-        if (S == 0) {
-            const double xp = tab[TB_X1 * kTabStride + j] * inv_kbt;
-            const double xe = xp * (kMe / kMp);
-            const double sum = coulomb_one(xe) + coulomb_one(xp) * (kMe / kMp);
-            const double thermal = 1.0 - kbt * tab[TB_X2 * kTabStride + j];
-            const double coul = (thermal < 0.0)
-                ? 0.0
-                : kGyr * kC / (kMp * kGeV) * sum * n_gas * tab[TB_X3 * kTabStride + j] * thermal * 3.5e-29;
-            radp = coul + adiab * p;
-        } else {
-            double r0, r1;
-            if (ric_stride == 0) {
-                r0 = tab[TB_X2 * kTabStride + j];
-                r1 = tab[TB_X3 * kTabStride + j];
-            } else {
-                r0 = ric[j * ric_stride];
-                r1 = ric_next[j * ric_stride];
-            }
-            const double r = interp ? lerp(r0, r1, alpha) : r0;
-            // log(p / n) as log p - log n: the per-bin logarithm is tabulated
-            const double coulomb = coulomb_coeff * (1.0 + (tab[TB_X1 * kTabStride + j] - log_n) * (1.0 / 74.8)) *
-                                   tab[TB_X0 * kTabStride + j];
-            radp = synch_coeff * p2 + r + coulomb + adiab * p;
-        }
-        B = radp - tab[TB_2P * kTabStride + j] * D;
-        C = D;
-    }
-
-    // dT = dt / tloss of row r of a lane's block (swizzled index r * kPitch + lane)
-    __device__ __forceinline__ double row_dT(const double *tab, int r, int lane) const
-    {
-        if (S == 0) return tab[TB_X4 * kTabStride + r * kPitch + lane] * dt_over_tloss_pref;
-        return dtT_e;
-    }
 };
 
-template <int S>
-__device__ __forceinline__ SegTerms<S> seg_terms(const GridTables &gt, const Bg &bg, int dis,
-                                                 const SnapArgs &a, const SegInfo &g, int t,
-                                                 int ic_stride)
+__device__ __forceinline__ SegTerms seg_terms(const Bg &bg, int dis, const SegInfo &g)
 {
-    SegTerms<S> T;
-    T.gt = &gt;
+    SegTerms T;
     T.n_gas = bg.n_gas;
     T.kbt = bg.kbt;
     T.inv_kbt = 1.0 / bg.kbt;
@@ -284,375 +191,680 @@ __device__ __forceinline__ SegTerms<S> seg_terms(const GridTables &gt, const Bg 
     T.dt = g.dt;
     T.dt_over_tloss_pref = g.dt / (1.0 / (0.5 * kC * bg.n_gas) / kGyr);
     T.dtT_e = g.dt / 1.0e+100;
-    T.ric = a.ic_curr + (ic_stride ? t : 0);
-    T.ric_next = a.ic_next + (ic_stride ? t : 0);
-    T.ric_stride = ic_stride;
     T.alpha = g.alpha;
     T.interp = g.nseg > 1;
-    T.dpp_inv = 0.0;
-    T.dpp_scale = 1.0;
-    T.dpp_fill = 0;
     return T;
 }
 
-// SegTerms of species S from the precomputed scalars of the segment.
-template <int S>
-__device__ __forceinline__ SegTerms<S> seg_terms_pre(const GridTables &gt, const SegPre *__restrict__ p,
-                                                     const SnapArgs &a, int t, int ic_stride)
+// Power-of-two factor that brings the larger of |x|, |y| into [1, 2) (1 where
+// that is zero, subnormal or not finite).
+__device__ __forceinline__ double pow2_norm(double x, double y)
 {
-    SegTerms<S> T;
-    T.gt = &gt;
-    T.n_gas = p->n_gas;
-    T.kbt = p->kbt;
-    T.inv_kbt = p->inv_kbt;
-    T.log_n = p->log_n;
-    T.adiab = p->adiab;
-    T.synch_coeff = p->synch_coeff;
-    T.coulomb_coeff = p->coulomb_coeff;
-    T.dt = p->dt;
-    T.dt_over_tloss_pref = p->dt_over_tloss_pref;
-    T.dtT_e = p->dtT_e;
-    T.ric = a.ic_curr + (ic_stride ? t : 0);
-    T.ric_next = a.ic_next + (ic_stride ? t : 0);
-    T.ric_stride = ic_stride;
-    T.alpha = p->alpha;
-    T.interp = (p->flags & kPreInterp) ? 1 : 0;
-    T.dpp_inv = 0.0;
-    T.dpp_scale = 1.0;
-    T.dpp_fill = 0;
-    return T;
+    const int ex = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >> 20;
+    return (ex <= 0 || ex >= 2046) ? 1.0 : __hiloint2double((2046 - ex) << 20, 0);
 }
 
-struct WarpSmem {
-    double B[kSw], C[kSw];
-    double Wp[kFacesInRegs ? 1 : kSw], Wm[kFacesInRegs ? 1 : kSw];
-};
-
-
-// Terms, faces and the rows a, b, c of one system: lane l holds rows
-// [l*R, (l+1)*R) in A, Bd, Cc.
-template <int S>
-__device__ unsigned build_rows(const SegTerms<S> &T, const double *tab, int lane, WarpSmem &sm,
-                               double A[kR], double Bd[kR], double Cc[kR])
+// The last two continuants before a lane's rows, from every lane's matrix of its
+// rows' recurrence (an exclusive scan over the LANES lanes of a system).
+template <int LANES>
+__device__ __forceinline__ void continuant_scan(double t00, double t01, double t10, double t11, int gl, double &th,
+                                                double &thp)
 {
-    const SpeciesTables &st = T.gt->s[S];
-    const double *x = st.p;
-    unsigned err = 0;
-
-    // Swizzled positions: for j = 32 k + lane, swz(j) = swz(lane) + k * 32 / R
-    // and swz(j + 1) = swz(lane + 1) + k * 32 / R; for row m = R lane + r of
-    // the lane's block, swz(m) = r * pitch + lane.
-    constexpr int kStep = 32 / kR;
-    const int sb0 = swz(lane), sb1 = swz(lane + 1);
-
-    // terms, lane-strided
-#pragma unroll 2
-    for (int k = 0; k < kR; k++) {
-        const int j = k * 32 + lane;
-        double B, C;
-        T.at(tab, j, B, C);
-        sm.B[sb0 + k * kStep] = B;
-        sm.C[sb0 + k * kStep] = C;
-    }
-    __syncwarp();
-    // Faces j (between bins j and j+1).  In registers (kFacesInRegs) where the
-    // rows use them: lane l's rows m = l R + r need faces m - 1 and m, so the
-    // lane evaluates faces l R - 1 .. l R + R - 1 (the first one its left
-    // neighbour evaluates too); else lane-strided into shared memory.  The
-    // drift / diffusion ratio
-    // (B_j + B_j+1) / (C_j + C_j+1) * dx: with the filled Dpp form the C sum
-    // is kappa times a grid factor, so the division becomes a product with the
-    // tabulated dx / (g_j + g_j+1) and 1 / kappa (equal to a few ulp).  The
-    // division form is taken only when a lane of the warp needs it (the vote
-    // keeps it from being computed predicated on every face).  Faces -1 and
-    // nb - 1 do not exist.
-    const double inv_kappa = T.dpp_fill ? 1.0 / (T.dpp_inv * T.dpp_scale) : 0.0;
-    auto face = [&](int j, int sj, int sj1, double &wp, double &wm) {
-        wp = 0.0;
-        wm = 0.0;
-        const bool exists = j >= 0 && j <= NB - 2;
-        const double cl = exists ? sm.C[sj] : 0.0;
-        const bool live = exists && fabs(cl) > 1.0e-200;
-        const double bsum = exists ? sm.B[sj] + sm.B[sj1] : 0.0;
-        const double rf = exists ? tab[TB_RF * kTabStride + sj] * inv_kappa : 0.0;
-        const bool divide = live && !(T.dpp_fill && isfinite(rf));
-        double w = bsum * rf;
-        if (__any_sync(kFull, divide)) {
-            if (divide) w = bsum / (cl + sm.C[sj1]) * tab[TB_DXF * kTabStride + sj];
-        }
-        if (live) face_weights_fast(w, wp, wm);
-    };
-
-    if (!kFacesInRegs) {
-        // faces lane-strided into shared memory (j = 32 k + lane); face nb - 1
-        // does not exist: its position swz(nb) is a padding word, never read
-#pragma unroll 2
-        for (int k = 0; k < kR; k++) {
-            const int j = k * 32 + lane;
-            const int s0 = sb0 + k * kStep, s1 = sb1 + k * kStep;
-            double wp = 0.0, wm = 0.0;
-            const double cl = sm.C[s0];
-            const bool live = (j <= NB - 2) && fabs(cl) > 1.0e-200;
-            const double bsum = sm.B[s0] + sm.B[s1];
-            const double rf = tab[TB_RF * kTabStride + j] * inv_kappa;
-            const bool divide = live && !(T.dpp_fill && isfinite(rf));
-            double w = bsum * rf;
-            if (__any_sync(kFull, divide)) {
-                if (divide) w = bsum / (cl + sm.C[s1]) * tab[TB_DXF * kTabStride + j];
-            }
-            if (live) face_weights_fast(w, wp, wm);
-            sm.Wp[kFacesInRegs ? 0 : s0] = wp;
-            sm.Wm[kFacesInRegs ? 0 : s0] = wm;
-        }
-        __syncwarp();
-    }
-
-    // rows a, b, c of this lane (cc_build_{left,interior,right}, Chang_Cooper.c:66-184)
-    const int row0 = lane * kR;
-    double wpm = 0.0, wmm = 0.0;   // face m - 1
-    if (kFacesInRegs) face(row0 - 1, lane > 0 ? (kR - 1) * kPitch + lane - 1 : 0, lane, wpm, wmm);
+    auto up = [](double v, int d) { return __shfl_up_sync(kFull, v, d, LANES); };
 #pragma unroll
-    for (int r = 0; r < kR; r++) {
-        const int m = row0 + r;
-        const int sm_m = r * kPitch + lane;
-        const int sm_p = r > 0 ? (r - 1) * kPitch + lane : (kR - 1) * kPitch + lane - 1;   // swz(m - 1), m >= 1
-        const int sm_n = r < kR - 1 ? (r + 1) * kPitch + lane : lane + 1;                  // swz(m + 1)
-        double wpc, wmc;   // face m
-        if (kFacesInRegs) {
-            face(m, sm_m, sm_n, wpc, wmc);
-        } else {
-            wpc = sm.Wp[kFacesInRegs ? 0 : sm_m];
-            wmc = sm.Wm[kFacesInRegs ? 0 : sm_m];
-            if (m > 0) {
-                wpm = sm.Wp[kFacesInRegs ? 0 : sm_p];
-                wmm = sm.Wm[kFacesInRegs ? 0 : sm_p];
-            }
+    for (int off = 1; off < LANES; off <<= 1) {
+        const double u00 = up(t00, off), u01 = up(t01, off), u10 = up(t10, off), u11 = up(t11, off);
+        if (gl >= off) {
+            const double n00 = fma(t00, u00, t01 * u10), n01 = fma(t00, u01, t01 * u11);
+            const double n10 = fma(t10, u00, t11 * u10), n11 = fma(t10, u01, t11 * u11);
+            t00 = n00; t01 = n01; t10 = n10; t11 = n11;
         }
-        const double k = T.dt * tab[TB_IDX * kTabStride + r * kPitch + lane];
-        const double Cm = sm.C[r * kPitch + lane], Bm = sm.B[r * kPitch + lane], Dm = T.row_dT(tab, r, lane);
-        double av = 0.0, bv, cv = 0.0;
-        if (m == 0) {
-            const double nC = sm.C[sm_n], nB = sm.B[sm_n];
-            if (fabs(Cm) > 1.0e-200) {
-                const double cm12 = 0.5 * (Cm + nC) * tab[TB_IDXR * kTabStride + r * kPitch + lane];
-                bv = 1.0 + k * (0.0 + cm12 * wmc) + Dm;
-                cv = k * cm12 * wpc;
-            } else {
-                bv = 1.0 + k * 0.0 + Dm;
-                cv = k * 1.0 * 0.5 * (Bm + nB);
-            }
-        } else {
-            const double pC = sm.C[sm_p], pB = sm.B[sm_p];
-            if (m == NB - 1) {
-                if (fabs(Cm) > 1.0e-200) {
-                    const double cm_12 = 0.5 * (Cm + pC) * tab[TB_IDXL * kTabStride + r * kPitch + lane];
-                    av = k * cm_12 * wmm;
-                    bv = 1.0 + k * (cm_12 * wpm) + Dm;
-                    if (isnan(av)) err |= kErrCcNan;
-                } else {
-                    double dlt = 0.0;
-                    if (fabs(pC) > 1.0e-200)
-                        dlt = face_delta((pB + Bm) / (pC + Cm) * (x[m] - x[m - 1]));
-                    av = -dlt * 0.5 * (Bm + pB) * k;
-                    bv = 1.0 + k * (0.5 * (pB + Bm)) + Dm;
-                }
-            } else {
-                const double nC = sm.C[sm_n], nB = sm.B[sm_n];
-                if (fabs(Cm) > 1.0e-200) {
-                    const double cm_12 = 0.5 * (Cm + pC) * tab[TB_IDXL * kTabStride + r * kPitch + lane];
-                    const double cm12 = 0.5 * (Cm + nC) * tab[TB_IDXR * kTabStride + r * kPitch + lane];
-                    av = k * cm_12 * wmm;
-                    bv = 1.0 + k * (cm_12 * wpm + cm12 * wmc) + Dm;
-                    cv = k * cm12 * wpc;
-                } else {
-                    // interior row below the diffusion floor: every delta the
-                    // reference reads here is zero (Chang_Cooper.c:91-103)
-                    bv = 1.0 + k * (0.5 * (Bm + pB)) + Dm;
-                    cv = k * 1.0 * 0.5 * (Bm + nB);
-                }
-            }
-        }
-        wpm = wpc;
-        wmm = wmc;
-        A[r] = av;
-        Bd[r] = bv;
-        Cc[r] = cv;
     }
-    __syncwarp();
-    return err;
+    th = up(t00, 1);
+    thp = up(t10, 1);
+    if (gl == 0) {
+        th = 1.0;
+        thp = 0.0;
+    }
 }
 
-// Thomas pivots of the rows a, b, c held as build_rows leaves them, in place:
-// Bd <- 1/d, A <- a/d, Cc <- c/d (0 on the last row), with
-// d_i = b_i + a_i c'_{i-1}, c'_i = -c_i / d_i (fp_thomas_solve_ws,
-// src/fp_shared_core.c:226-257).  The chain of Moebius maps d -> b - e/d is
-// composed per lane as 2x2 matrices and combined by a warp scan, after which
-// each lane re-runs the exact recurrence on its rows from the scanned
-// incoming pivot.  The lane's own matrix is rescaled to a largest entry in
-// [1, 2); the scan's products then stay below 2^63 over its five levels, so
-// they are not rescaled (powers of two are exact either way: same pivots).
-__device__ __forceinline__ unsigned pivot_rows(double A[kR], double Bd[kR], double Cc[kR], int lane)
+// |theta_i / theta_{i-1}| <= 1e-300, to its exponent
+__device__ __forceinline__ bool continuant_singular(double n, double th)
 {
+    return (__double2hiint(n) & 0x7fffffff) + (996 << 20) < (__double2hiint(th) & 0x7fffffff);
+}
+
+// Thomas pivots of the rows a, b, c of a system, in place: Bd <- 1/d, A <- a/d,
+// Cc <- c/d, with d_i = b_i - a_i c_{i-1} / d_{i-1} (fp_thomas_solve_ws,
+// src/fp_shared_core.c:226-257); R rows a lane, LANES lanes a system, gl the
+// lane's place among them.  The pivots are ratios of continuants, d_i = theta_i
+// / theta_{i-1} with theta_i = b_i theta_{i-1} - e_i theta_{i-2}, e_i = a_i
+// c_{i-1}: each lane forms the 2x2 matrix of its rows' recurrence (rescaled by
+// exact powers of two to a largest entry in [1, 2); the scan's products stay
+// below 2^63), a scan over the lanes gives it its incoming pair, and it runs the
+// recurrence on its rows from there.  One FMA a row is all that is serial: the
+// reciprocals theta_{i-1} / theta_i are independent of each other, where the
+// pivot recurrence itself waits for one reciprocal a row (66 cycles against 8).
+// A row's rounding errors are those of d = b - e / d, since only the ratio of
+// the last two continuants enters it.
+template <int R, int LANES>
+__device__ __forceinline__ unsigned pivot_rows(double A[R], double Bd[R], double Cc[R], int gl)
+{
+    auto up = [](double v, int d) { return __shfl_up_sync(kFull, v, d, LANES); };
     unsigned err = 0;
-    const int row0 = lane * kR;
-    const double c_in = sup(Cc[kR - 1], 1);   // c of the row before this lane's first
+    double c_in = up(Cc[R - 1], 1);   // c of the row before this lane's first
+    c_in = gl > 0 ? c_in : 0.0;
     double t00 = 1.0, t01 = 0.0, t10 = 0.0, t11 = 1.0;
 #pragma unroll
-    for (int r = 0; r < kR; r++) {
-        const double cprev = (r > 0) ? Cc[r - 1] : (lane > 0 ? c_in : 0.0);
-        const double e = A[r] * cprev;
-        const double n00 = Bd[r] * t00 - e * t10;
-        const double n01 = Bd[r] * t01 - e * t11;
+    for (int r = 0; r < R; r++) {
+        const double e = A[r] * (r > 0 ? Cc[r - 1] : c_in);
+        const double n00 = fma(Bd[r], t00, -(e * t10));
+        const double n01 = fma(Bd[r], t01, -(e * t11));
         t10 = t00;
         t11 = t01;
         t00 = n00;
         t01 = n01;
-        if ((r & 3) == 3) rescale2(t00, t01, t10, t11);
-    }
-    rescale2(t00, t01, t10, t11);
-#pragma unroll
-    for (int lv = 0; lv < 5; lv++) {
-        const int off = 1 << lv;
-        const double u00 = sup(t00, off), u01 = sup(t01, off), u10 = sup(t10, off), u11 = sup(t11, off);
-        if (lane >= off) {
-            const double n00 = t00 * u00 + t01 * u10, n01 = t00 * u01 + t01 * u11;
-            const double n10 = t10 * u00 + t11 * u10, n11 = t10 * u01 + t11 * u11;
-            t00 = n00; t01 = n01; t10 = n10; t11 = n11;
+        if ((r & 7) == 7 || r == R - 1) {   // d < 2^127 cannot leave the range in eight rows
+            const double sc = pow2_norm(t00, t01);
+            t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
         }
     }
-    double vp = sup(t00, 1), vq = sup(t10, 1);
-    double cp_prev = (lane == 0) ? 0.0 : -c_in * vq * rcp_nr(vp);
+    double th, thp;
+    continuant_scan<LANES>(t00, t01, t10, t11, gl, th, thp);
+    double cprev = c_in;
 #pragma unroll
-    for (int r = 0; r < kR; r++) {
-        const int m = row0 + r;
-        const double den = Bd[r] + A[r] * cp_prev;
-        if (fabs(den) <= 1.0e-300) err |= kErrSingular;
-        const double inv = rcp_nr(den);
-        const double cr = Cc[r];
+    for (int r = 0; r < R; r++) {
+        const double n = fma(Bd[r], th, -(A[r] * cprev * thp));
+        if (continuant_singular(n, th)) err = kErrSingular;
+        const double inv = th * rcp_nr(n);
+        cprev = Cc[r];
         Bd[r] = inv;
-        A[r] = A[r] * inv;
-        Cc[r] = (m == NB - 1) ? 0.0 : cr * inv;
-        cp_prev = -cr * inv;
+        A[r] *= inv;
+        Cc[r] *= inv;
+        thp = th;
+        th = n;
+        if ((r & 7) == 7 && r < R - 1) {
+            const double sc = pow2_norm(th, thp);
+            th *= sc;
+            thp *= sc;
+        }
     }
-    (void)vp;
     return err;
 }
 
-// Three row arrays of a lane to out[0..3nb): R contiguous doubles per array
-// per lane (32-byte stores), nb doubles per array per warp.
-__device__ __forceinline__ void store_rows(double *out, int lane, const double X[kR], const double Y[kR],
-                                           const double Z[kR])
+// Sixteen (eight) 32-bit TMEM columns of the warp's lanes.  The loads are
+// asynchronous: the registers are valid after tmem_wait, which names them so
+// that no use is scheduled before it (tmem_after8: a further load that the same
+// wait covers).
+struct Tmem16 {
+    unsigned r[16];
+    __device__ __forceinline__ double d(int i) const { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
+};
+__device__ __forceinline__ void tmem_ld16(unsigned t, Tmem16 &u)
 {
-    const int row0 = lane * kR;
-#pragma unroll
-    for (int r = 0; r < kR; r += 4) {
-        st4_cg(out + row0 + r, X + r);
-        st4_cg(out + NB + row0 + r, Y + r);
-        st4_cg(out + 2 * NB + row0 + r, Z + r);
-    }
+    unsigned *r = u.r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(t));
+}
+__device__ __forceinline__ void tmem_ld8(unsigned t, unsigned *r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(t));
+}
+__device__ __forceinline__ void tmem_wait(Tmem16 &u)
+{
+    unsigned *r = u.r;
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
+}
+__device__ __forceinline__ void tmem_after8(unsigned *r)
+{
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+}
+__device__ __forceinline__ void tmem_wait8(unsigned *r)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+}
+__device__ __forceinline__ void tmem_st8(unsigned t, const unsigned *r)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 
-// One system of species S to out: factored (1/d, a/d, c/d) for the steps
-// kernel, or the raw rows (a, b, c) for the per-step path, which factors
-// them again on every sub-step.
-template <int S, bool ROWS>
-__device__ unsigned factor_store(const SegTerms<S> &T, const double *tab, int lane, WarpSmem &sm,
-                                 double *out)
+__device__ __forceinline__ void pk_set(unsigned *r, int i, double v)
 {
-    double A[kR], Bd[kR], Cc[kR];
-    unsigned err = build_rows<S>(T, tab, lane, sm, A, Bd, Cc);
-    if (ROWS) {
-        store_rows(out, lane, A, Bd, Cc);
-        return err;
+    r[2 * i] = (unsigned)__double2loint(v);
+    r[2 * i + 1] = (unsigned)__double2hiint(v);
+}
+__device__ __forceinline__ double pk_get(const unsigned *r, int i) { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
+
+// TMEM columns of a block, its base address through shared memory; one warp of
+// the block calls each.  The allocation waits until the SM has the columns,
+// which the blocks that hold them give back when they end.
+template <int COLUMNS>
+__device__ __forceinline__ void tmem_alloc(unsigned *base)
+{
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(base)),
+                 "n"(COLUMNS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+template <int COLUMNS>
+__device__ __forceinline__ void tmem_free(unsigned base)
+{
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLUMNS));
+}
+__device__ __forceinline__ void tmem_st2(unsigned t, double v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(t), "r"(__double2loint(v)),
+                 "r"(__double2hiint(v))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
+// Factor kernel, persistent: a block stages the species' grid tables once, in
+// the packed layout (lane gl holds rows 16 gl .. 16 gl + 15 of its system; the
+// systems of a warp are neighbouring segments and sets of one tracer), and its
+// warps take units of kPkTracers systems in turn, the next unit's scalars
+// copied to shared memory meanwhile.
+//
+// It is bound by the latency of its FP64 instructions, exponentials and
+// reciprocals.  So their number is kept down: what depends on the grid alone
+// is tabulated -- with the diffusion coefficient kappa g(p), g = p^2 exp(-1/p)
+// (protons: times exp(-E/E_max)) and kappa the segment's 1 / (4 t_acc) times
+// the eta cap's scale, or the "off" form g = p^2, kappa = 1 / (4e5), a face
+// needs 2 g / p, dx / (g_j + g_j+1) and (g_j + g_j+1) / (2 dx) -- and each face
+// is evaluated once: the row above takes it from the lane's registers or its
+// neighbour's.  And the rows wait in tensor memory between the face loop, which
+// also runs the continuants' recurrence, and the second pass (pivot_rows'
+// arithmetic): 128 registers, 16 warps per SM.  The face loop is unrolled by four
+// rows only, so that it stays in the instruction cache.  Rows with a vanishing
+// diffusion coefficient (kappa g <= 1e-200) have their own forms
+// (Chang_Cooper.c:66-184); a system that could meet them takes rows_general.
+//
+// Measured, before (a warp per system at every bin count, coefficients staged
+// in shared memory, a reciprocal a row in the serial chain of the pivots) and
+// now, protons and electrons: 512 bins, 131,072 tracers x 16 segments 20.6 and
+// 16.7 -> 11.2 and 9.0 ms; 256 bins, 65,536 tracers 3.82 and 3.18 -> 2.93 and
+// 2.25 ms; 128 bins, 131,072 tracers (electrons) 3.53 -> 2.25 ms; 64 tracers 61
+// -> 13 us.  12 warps with the rows in registers 12.5 and 11.2 ms at 512 bins,
+// the face loop unrolled whole 12.4 and 9.9.  FP64 pipe 45 %.
+// Tables are pairs of doubles, read 16 bytes at a time:
+enum { FT_X01,      // electrons: p^2, 1/beta^2;  protons: 1/beta^2, that / (2 m_p (gamma - 1))
+       FT_X2P,      // electrons: log p / beta^2, p;  protons: sig_eff, p
+       FT_X34,      // electrons: IC row at z_curr, its change to z_next;  protons: gamma m_p - m_p of two bins, grid order
+       FT_GR,       // filled Dpp form: 2 g / p, dx / (g_j + g_j+1)
+       FT_FK,       //                  (g_j + g_j+1) / (2 dx), 1 / dp
+       FT_OFF,      // the same two of the off form
+       kFacTabs = FT_OFF + 2 };
+constexpr int kFacWarps = 8;
+constexpr int kFacBlocks = 2;      // blocks per SM
+constexpr int kFacColumns = 256;   // TMEM: two warps a lane quarter, 96 of 128 columns each
+// Protons: the Coulomb kernel of a warp's systems, lane-strided (so that the
+// bins that need its erf and exp are whole warps), read back packed: row r of
+// lane gl at r * kCoulPitch + gl, an odd pitch for distinct banks.
+constexpr int kCoulPitch = kPkLanes + 1;
+constexpr int kCoulSys = kPkRows * kCoulPitch;
+constexpr int kCoulWarp = kPkTracers * kCoulSys;
+
+// Chang-Cooper weights of a face (face_weights_fast's arithmetic, with one
+// exponential exp(-|w| / 2) for both of its branches).
+__device__ __forceinline__ void face_weights_half(double w, double &wp, double &wm)
+{
+    const double aw = fabs(w);
+    const bool series = aw < 0.1;
+    // exp(-700) squared is 0, as exp(-1400) is (a NaN comes through aw below)
+    const double E = exp_tab_normal(aw < 1400.0 ? -0.5 * aw : -700.0);
+    const double e2 = E * E, w2 = w * w;
+    const double dser = fma(w2, fma(w2, 1.0 / 1920.0, 1.0 / 24.0), 1.0);
+    const double q = (series ? 1.0 : aw) * rcp_nr(series ? E * dser : 1.0 - e2);
+    const double s = q * e2;
+    wp = (w >= 0.0) ? q : s;
+    wm = (w >= 0.0) ? s : q;
+}
+
+// B = radp - 2 Dpp / p and C = Dpp at bin j, straight from the grid tables.
+template <int S>
+__device__ double2 terms_general(const FusedParams &P, const SegPre &p, double alpha, bool fill, double scale, int t, int j)
+{
+    const SpeciesTables &st = P.gt.s[S];
+    const double x = st.p[j];
+    double D = st.p2[j] * (1.0 / (4.0 * 1.0e+5));
+    if (fill) D = S == 0 ? st.p2[j] * p.dpp_inv * st.expE[j] * st.exp_cut[j] : st.p2[j] * p.dpp_inv * st.exp_cut[j];
+    D *= scale;
+    double radp;
+    if (S == 0) {
+        const double xp = P.gt.cp_Ep[j] * p.inv_kbt;
+        const double sum = coulomb_one(xp * (kMe / kMp)) + coulomb_one(xp) * (kMe / kMp);
+        const double thermal = 1.0 - p.kbt * P.gt.cp_inv2mpkin[j];
+        radp = (thermal < 0.0 ? 0.0
+                              : kGyr * kC / (kMp * kGeV) * sum * p.n_gas * P.gt.cp_inv_betap2[j] * thermal * 3.5e-29) +
+               p.adiab * x;
+    } else {
+        const size_t at = P.ic_stride ? (size_t)j * P.ic_stride + t : (size_t)j;
+        radp = p.synch_coeff * st.p2[j] + lerp(P.a.ic_curr[at], P.a.ic_next[at], alpha) +
+               p.coulomb_coeff * (1.0 + (P.gt.ce_logp[j] - p.log_n) * (1.0 / 74.8)) * P.gt.ce_inv_beta2[j] + p.adiab * x;
     }
-    err |= pivot_rows(A, Bd, Cc, lane);
-    store_rows(out, lane, Bd, A, Cc);
+    return make_double2(radp - st.two_over_p[j] * D, D);
+}
+
+// The raw rows a, b, c of the lane's 16 rows to out, with the forms of rows
+// and faces whose diffusion coefficient vanishes (cc_build_{left,interior,
+// right}, Chang_Cooper.c:66-184).  Rolled and slow: for systems that can meet
+// them only.
+template <int S>
+__device__ __noinline__ unsigned rows_general(const FusedParams &P, const SegPre &p, double alpha, bool fill, double scale,
+                                              int t, int gl, double *out)
+{
+    const SpeciesTables &st = P.gt.s[S];
+    unsigned err = 0;
+    auto face = [&](double2 l, double2 r, int j, double &wp, double &wm) {   // face j, between bins j and j + 1
+        wp = wm = 0.0;
+        if (fabs(l.y) > 1.0e-200) face_weights_fast((l.x + r.x) / (l.y + r.y) * st.dxf[j], wp, wm);
+    };
+#pragma unroll 1
+    for (int r = 0; r < kPkRows; r++) {
+        const int m = gl * kPkRows + r;
+        const double2 c0 = terms_general<S>(P, p, alpha, fill, scale, t, m);
+        const double2 cm = m > 0 ? terms_general<S>(P, p, alpha, fill, scale, t, m - 1) : make_double2(0.0, 0.0);
+        const double2 cp = m < NB - 1 ? terms_general<S>(P, p, alpha, fill, scale, t, m + 1) : make_double2(0.0, 0.0);
+        double wpm = 0.0, wmm = 0.0, wpc = 0.0, wmc = 0.0;
+        if (m > 0) face(cm, c0, m - 1, wpm, wmm);
+        if (m < NB - 1) face(c0, cp, m, wpc, wmc);
+        const double k = p.dt * st.inv_dx[m], D = S == 0 ? P.gt.sig_eff[m] * p.dt_over_tloss_pref : p.dtT_e;
+        const bool live = fabs(c0.y) > 1.0e-200;
+        double av = 0.0, bv, cv = 0.0;
+        const double fl = m > 0 ? 0.5 * (c0.y + cm.y) * st.inv_dxl[m] : 0.0;
+        const double fr = m < NB - 1 ? 0.5 * (c0.y + cp.y) * st.inv_dxr[m] : 0.0;
+        if (live) {
+            av = k * fl * wmm;
+            bv = 1.0 + k * (fl * wpm + fr * wmc) + D;
+            cv = k * fr * wpc;
+            if (m == NB - 1 && isnan(av)) err |= kErrCcNan;
+        } else if (m == 0) {
+            bv = 1.0 + k * 0.0 + D;
+            cv = k * 1.0 * 0.5 * (c0.x + cp.x);
+        } else if (m == NB - 1) {
+            double dlt = 0.0;
+            if (fabs(cm.y) > 1.0e-200) dlt = face_delta((cm.x + c0.x) / (cm.y + c0.y) * (st.p[m] - st.p[m - 1]));
+            av = -dlt * 0.5 * (c0.x + cm.x) * k;
+            bv = 1.0 + k * (0.5 * (cm.x + c0.x)) + D;
+        } else {
+            // every delta the reference reads here is zero (Chang_Cooper.c:91-103)
+            bv = 1.0 + k * (0.5 * (c0.x + cm.x)) + D;
+            cv = k * 1.0 * 0.5 * (c0.x + cp.x);
+        }
+        __stcg(out + m, av);
+        __stcg(out + NB + m, bv);
+        __stcg(out + 2 * NB + m, cv);
+    }
     return err;
 }
 
-
-// Factor kernel, persistent: each block stages the species' grid tables in
-// shared memory once, then each warp takes tracers strided by the grid and
-// factors every segment (and on/off set) of each (ROWS: stores the raw rows).
+// ROWS: stores the raw rows a, b, c for the per-step path, which factors them
+// again on every sub-step; else the factored 1/d, a/d, c/d.
 template <int S, bool ROWS>
-__global__ void __launch_bounds__(kFacWarps * 32, (NB <= 256 ? 2 : 1)) factor_kernel(FusedParams P)
+__global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(const __grid_constant__ FusedParams P)
 {
+    constexpr int R = kPkRows, G = kPkLanes;
     extern __shared__ double4 smem_raw[];
-    double *tab = reinterpret_cast<double *>(smem_raw);
-    WarpSmem *smem = reinterpret_cast<WarpSmem *>(tab + kTab * kTabStride);
-    const int w = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
+    double2 *tab = reinterpret_cast<double2 *>(smem_raw);
+    __shared__ double g_warp[2][kFacWarps];        // least g of the filled and the off form, per warp's share
+    __shared__ SegPre pre_next[2][kFacWarps * kPkTracers];   // scalars of the warp's systems, one unit ahead
+    static_assert(sizeof(SegPre) == 7 * 16 && G >= 7, "a group's lanes copy its SegPre 16 bytes each");
+    __shared__ unsigned tmem_base;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (G - 1);
+    if (w == 0) tmem_alloc<kFacColumns>(&tmem_base);
     const SnapArgs &a = P.a;
     const SpeciesTables &st = P.gt.s[S];
+    auto g_of = [&](int form, int i) {
+        return form ? st.p2[i] : (S == 0 ? st.p2[i] * st.expE[i] * st.exp_cut[i] : st.p2[i] * st.exp_cut[i]);
+    };
+    double g_min[2] = {1.0e+308, 1.0e+308};
     for (int i = threadIdx.x; i < NB; i += blockDim.x) {
-        tab[TB_P * kTabStride + i] = st.p[i];
-        tab[TB_P2 * kTabStride + i] = st.p2[i];
-        tab[TB_CUT * kTabStride + i] = st.exp_cut[i];
-        tab[TB_2P * kTabStride + i] = st.two_over_p[i];
-        tab[TB_DXF * kTabStride + (kFacesInRegs ? swz(i) : i)] = st.dxf[i];
-        tab[TB_RF * kTabStride + (kFacesInRegs ? swz(i) : i)] = st.face_rf[i];
+        const int at = (i % R) * G + i / R;
         if (S == 0) {
-            tab[TB_X0 * kTabStride + i] = st.expE[i];
-            tab[TB_X1 * kTabStride + i] = P.gt.cp_Ep[i];
-            tab[TB_X2 * kTabStride + i] = P.gt.cp_inv2mpkin[i];
-            tab[TB_X3 * kTabStride + i] = P.gt.cp_inv_betap2[i];
-            tab[TB_X4 * kTabStride + swz(i)] = P.gt.sig_eff[i];
+            tab[FT_X01 * NB + at] = make_double2(P.gt.cp_inv_betap2[i], P.gt.cp_inv_betap2[i] * P.gt.cp_inv2mpkin[i]);
+            tab[FT_X2P * NB + at] = make_double2(P.gt.sig_eff[i], st.p[i]);
+            reinterpret_cast<double *>(tab + FT_X34 * NB)[i] = P.gt.cp_Ep[i];
         } else {
-            tab[TB_X0 * kTabStride + i] = P.gt.ce_inv_beta2[i];
-            tab[TB_X1 * kTabStride + i] = P.gt.ce_logp[i];
-            tab[TB_X2 * kTabStride + i] = (P.ic_stride == 0) ? a.ic_curr[i] : 0.0;
-            tab[TB_X3 * kTabStride + i] = (P.ic_stride == 0) ? a.ic_next[i] : 0.0;
-            tab[TB_X4 * kTabStride + swz(i)] = 0.0;
+            const double r0 = P.ic_stride == 0 ? a.ic_curr[i] : 0.0;
+            tab[FT_X01 * NB + at] = make_double2(st.p2[i], P.gt.ce_inv_beta2[i]);
+            tab[FT_X2P * NB + at] = make_double2(P.gt.ce_logp[i] * P.gt.ce_inv_beta2[i], st.p[i]);
+            tab[FT_X34 * NB + at] = make_double2(r0, P.ic_stride == 0 ? a.ic_next[i] - r0 : 0.0);
         }
-        tab[TB_IDX * kTabStride + swz(i)] = st.inv_dx[i];
-        tab[TB_IDXL * kTabStride + swz(i)] = st.inv_dxl[i];
-        tab[TB_IDXR * kTabStride + swz(i)] = st.inv_dxr[i];
+#pragma unroll
+        for (int form = 0; form < 2; form++) {
+            const double g = g_of(form, i);
+            const bool face = i < NB - 1;   // the last bin has no face above: weights of a zero flux
+            const double gs = face ? g + g_of(form, i + 1) : 0.0;
+            tab[(FT_GR + 2 * form) * NB + at] = make_double2(st.two_over_p[i] * g, face ? st.dxf[i] / gs : 0.0);
+            tab[(FT_FK + 2 * form) * NB + at] = make_double2(face ? 0.5 * gs * st.inv_dxr[i] : 0.0, st.inv_dx[i]);
+            g_min[form] = fmin(g_min[form], g);
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        g_min[0] = fmin(g_min[0], __shfl_xor_sync(kFull, g_min[0], off));
+        g_min[1] = fmin(g_min[1], __shfl_xor_sync(kFull, g_min[1], off));
+    }
+    if (lane == 0) {
+        g_warp[0][w] = g_min[0];
+        g_warp[1][w] = g_min[1];
     }
     __syncthreads();
-    // a warp takes one tracer at a time and factors all its segments (and
-    // on/off sets) from the segments' precomputed scalars; after its first
-    // tracer it takes the next one not yet taken (a counter the host zeroes
-    // before the launch), so no warp is left with a whole extra tracer at the end
-    const int stride = gridDim.x * kFacWarps;
-    const int nslot = P.g1 - P.g0;
-    int tl = blockIdx.x * kFacWarps + w;
+#pragma unroll
+    for (int k = 0; k < kFacWarps; k++) {
+        g_min[0] = fmin(g_min[0], g_warp[0][k]);
+        g_min[1] = fmin(g_min[1], g_warp[1][k]);
+    }
+    // rows a, b, c of chunk k (four rows) of the warp's lanes: 8 columns each
+    const unsigned tm = tmem_base + ((unsigned)((w & 3) * 32) << 16) + (w >> 2) * 128;
+    // A unit: kPkTracers (segment, set) pairs of one tracer, or, with fewer pairs
+    // than that, those of several tracers; unit numbers run over the tracers
+    // first, so that pairs beyond a tracer's last segment fall evenly on the warps.
+    const int per = (P.g1 - P.g0) * P.sets, pairs = min(per, kPkTracers), tracers = kPkTracers / pairs;
+    const int nq = (P.nt + tracers - 1) / tracers;
+    const int units = (per + pairs - 1) / pairs * nq, stride = gridDim.x * kFacWarps;
+    const int sub = (lane / G) / pairs, off = (lane / G) - sub * pairs;   // the group's place in the unit
+    double *coul = reinterpret_cast<double *>(tab + kFacTabs * NB) + w * kCoulWarp;
+    const double2 *row = tab + gl;                // table k, row r of the lane: row[k * NB + r * G]
+    const int group = w * kPkTracers + lane / G;
+    auto locate = [&](int unit, int &tl, int &gi, int &set) {
+        const int blk = unit / nq, slot = blk * pairs + off;
+        tl = (unit - blk * nq) * tracers + sub;
+        gi = slot / P.sets;
+        set = slot - gi * P.sets;
+        return unit < units && sub < tracers && tl < P.nt && slot < per;
+    };
+    auto fetch = [&](int unit, int buf) {         // the unit's scalars, 16 bytes a lane
+        int tl, gi, set;
+        if (locate(unit, tl, gi, set) && gl < 7)
+            cp_async16(reinterpret_cast<char *>(&pre_next[buf][group]) + 16 * gl,
+                       reinterpret_cast<const char *>(P.pre + (size_t)gi * P.nt + tl) + 16 * gl, true);
+    };
+    int buf = 1;
+    fetch(blockIdx.x * kFacWarps + w, 0);
 #pragma unroll 1
-    while (tl < P.nt) {
+    for (int unit = blockIdx.x * kFacWarps + w; unit < units; unit += stride) {
+        int tl, gi, set;
+        const bool here = locate(unit, tl, gi, set);
+        if (!here) tl = gi = set = 0;
+        buf ^= 1;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        fetch(unit + stride, buf ^ 1);
         const int t = P.t0 + tl;
-        WarpSmem &ws = smem[w];
-        const double eta = (P.mp.dpp_model != kDppOff && P.eta_scale) ? P.eta_scale[t] : 1.0;
-#pragma unroll 1
-        for (int gi = 0; gi < nslot; gi++) {
-            const SegPre *__restrict__ pre = P.pre + (size_t)gi * P.nt + tl;
-            const int flags = pre->flags;
-            if (!(flags & kPreActive)) break;
-            SegInfo g{};
-            g.windowed = (flags & kPreWindowed) ? 1 : 0;
-            g.sl = pre->sl;
-            g.el = pre->el;
-            g.steps = pre->steps;
-            if (needs_set(g, 1) && P.sets < 2) {   // checked on the host; never write past the sets
-                if (lane == 0) atomicOr(a.err, kErrBadInput);
-                continue;
+        const SegPre &pre = pre_next[buf][group];
+        const int flags = here ? pre.flags : 0;
+        SegInfo si{};
+        si.windowed = (flags & kPreWindowed) ? 1 : 0;
+        si.sl = pre.sl;
+        si.el = pre.el;
+        si.steps = pre.steps;
+        bool on = (flags & kPreActive) && needs_set(si, set);
+        if (on && needs_set(si, 1) && P.sets < 2) {   // checked on the host; never write past the sets
+            if (gl == 0) atomicOr(a.err, kErrBadInput);
+            on = false;
+        }
+        if (!__any_sync(kFull, on)) continue;
+        const bool fill = set == 0 && (flags & kPreFill);
+        const double scale = (set == 0 && P.mp.dpp_model != kDppOff && P.eta_scale) ? P.eta_scale[t] : 1.0;
+        const double kappa = fill ? pre.dpp_inv * scale : (1.0 / (4.0 * 1.0e+5)) * scale;
+        const double inv_kappa = 1.0 / kappa;
+        const double alpha = (flags & kPreInterp) ? pre.alpha : 0.0;
+        const double g_lo = g_min[fill ? 0 : 1];
+        const bool general = on && !(g_lo > 1.0e-290 && kappa * g_lo > 1.0e-200 && isfinite(kappa) && isfinite(inv_kappa));
+        const double dt = pre.dt, adiab = pre.adiab;
+        double *out = fac_ptr(P, S, gi, set, tl);
+        unsigned err = 0;
+        // per-bin scalars of B
+        double s0, s1, s2;
+        if (S == 0) {
+            s0 = kGyr * kC / (kMp * kGeV) * 3.5e-29 * pre.n_gas;
+            s1 = pre.kbt;
+            s2 = pre.dt_over_tloss_pref;
+            // the Coulomb kernels of the warp's systems
+#pragma unroll 2
+            for (int it = 0; it < R; it++) {
+                const int i = it * 32 + lane, sys = i / NB, j = i % NB;
+                const double ik = __shfl_sync(kFull, pre.inv_kbt, sys * G);
+                const double xp = reinterpret_cast<const double *>(tab + FT_X34 * NB)[j] * ik;
+                const double sum = coulomb_one(xp * (kMe / kMp)) + coulomb_one(xp) * (kMe / kMp);
+                coul[sys * kCoulSys + (j % R) * kCoulPitch + j / R] = sum;
             }
-#pragma unroll 1
-            for (int set = 0; set < P.sets; set++) {
-                if (!needs_set(g, set)) continue;
-                SegTerms<S> T = seg_terms_pre<S>(P.gt, pre, a, t, P.ic_stride);
-                if (set == 0) {
-                    T.dpp_fill = (flags & kPreFill) ? 1 : 0;
-                    T.dpp_inv = pre->dpp_inv;
-                    T.dpp_scale = eta;
+            __syncwarp();
+        } else {
+            s0 = pre.synch_coeff;
+            s1 = pre.coulomb_coeff * (1.0 - pre.log_n * (1.0 / 74.8));
+            s2 = pre.coulomb_coeff * (1.0 / 74.8);
+        }
+        const double2 *form = row + (fill ? 0 : 2 * NB);
+        const double *cs = coul + (lane / G) * kCoulSys + gl;
+        const double al = alpha <= 0.0 ? 0.0 : (alpha >= 1.0 ? 1.0 : alpha);
+        auto B_of = [&](int r, double g2p) {
+            const double2 x01 = row[FT_X01 * NB + r * G], x2p = row[FT_X2P * NB + r * G];
+            double B;
+            if (S == 0) {
+                const double ct = fma(-s1, x01.y, x01.x);
+                B = s0 * cs[r * kCoulPitch] * (ct < 0.0 ? 0.0 : ct);
+            } else {
+                double ric;
+                if (P.ic_stride == 0) {
+                    const double2 x34 = row[FT_X34 * NB + r * G];
+                    ric = fma(al, x34.y, x34.x);
+                } else {
+                    const size_t at = (size_t)(gl * R + r) * P.ic_stride + t;
+                    ric = lerp(a.ic_curr[at], a.ic_next[at], alpha);
                 }
-                const unsigned err = factor_store<S, ROWS>(T, tab, lane, ws, fac_ptr(P, S, gi, set, tl));
-                if (err && lane == 0) atomicOr(a.err, err);
+                B = fma(s0, x01.x, ric);
+                B = fma(s1, x01.y, B);
+                B = fma(s2, x2p.x, B);
+            }
+            B = fma(adiab, x2p.y, B);
+            return fma(-kappa, g2p, B);
+        };
+        // Rows from the faces above them (cc_build_*, Chang_Cooper.c:66-184), into
+        // TMEM, and the matrix of the continuants' recurrence over rows 1 .. 15.
+        // A lane's first row waits for its neighbour's last face.
+        double t00 = 1.0, t01 = 0.0, t10 = 0.0, t11 = 1.0;
+        double a0, b0, c0, e1 = 0.0;
+        {
+            double2 gr = form[FT_GR * NB];
+            double Bc = B_of(0, gr.x), Pl = 0.0, Ml = 0.0, cl = 0.0;   // flux times weights of the face below; c of the row below
+            const double B_up = __shfl_down_sync(kFull, Bc, 1, G);
+#pragma unroll 1
+            for (int kk = 0; kk < R / 4; kk++) {
+                unsigned ua[8], ub[8], uc[8];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = 4 * kk + i;
+                    const double rf = gr.y;
+                    double Bn = B_up;
+                    if (r < R - 1) {
+                        gr = form[FT_GR * NB + (r + 1) * G];
+                        Bn = B_of(r + 1, gr.x);
+                    }
+                    const double2 fk = form[FT_FK * NB + r * G];
+                    double wp, wm;
+                    face_weights_half((Bc + Bn) * (rf * inv_kappa), wp, wm);
+                    const double F = kappa * fk.x;
+                    const double Pu = F * wp, Mu = F * wm;
+                    const double k = dt * fk.y;
+                    const double D = S == 0 ? row[FT_X2P * NB + r * G].x * s2 : pre.dtT_e;
+                    const double ar = k * Ml, br = 1.0 + k * (Pl + Mu) + D, cr = k * Pu;
+                    pk_set(ua, i, ar);
+                    pk_set(ub, i, br);
+                    pk_set(uc, i, cr);
+                    if (r == 0) {
+                        b0 = br;
+                        c0 = cr;
+                    } else {
+                        const double e = ar * cl;
+                        const double n00 = fma(br, t00, -(e * t10)), n01 = fma(br, t01, -(e * t11));
+                        t10 = t00;
+                        t11 = t01;
+                        t00 = n00;
+                        t01 = n01;
+                        if (r == 7) {   // d < 2^127 cannot leave the range in eight rows
+                            const double sc = pow2_norm(t00, t01);
+                            t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
+                        }
+                        if (r == R - 1 && gl == G - 1 && on && !general && isnan(ar)) err |= kErrCcNan;
+                    }
+                    cl = cr;
+                    Bc = Bn;
+                    Pl = Pu;
+                    Ml = Mu;
+                }
+                tmem_st8(tm + kk * 24, ua);
+                tmem_st8(tm + kk * 24 + 8, ub);
+                tmem_st8(tm + kk * 24 + 16, uc);
+            }
+            Pl = __shfl_up_sync(kFull, Pl, 1, G);
+            Ml = __shfl_up_sync(kFull, Ml, 1, G);
+            const double k0 = dt * form[FT_FK * NB].y;
+            a0 = gl > 0 ? k0 * Ml : 0.0;
+            b0 = gl > 0 ? fma(k0, Pl, b0) : b0;
+            tmem_wait_st();   // chunk 0 is there before two of its columns are written again
+            tmem_st2(tm, a0);
+            tmem_st2(tm + 8, b0);
+            e1 = __shfl_up_sync(kFull, cl, 1, G);   // c of the row below the lane's first
+        }
+        if (__any_sync(kFull, general)) {
+            // those systems' rows by their own forms, through the output slot
+            if (general) err |= rows_general<S>(P, pre, alpha, fill, scale, t, gl, out);
+            __syncwarp();
+            tmem_wait_st();
+#pragma unroll 1
+            for (int r = 0; r < R; r++) {
+                double v[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const unsigned col = tm + (r >> 2) * 24 + 8 * k + 2 * (r & 3);
+                    unsigned q0, q1;
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(q0), "=r"(q1) : "r"(col));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(q0), "+r"(q1));
+                    v[k] = __hiloint2double((int)q1, (int)q0);
+                    if (general) v[k] = __ldcg(out + k * NB + gl * R + r);
+                    __syncwarp();
+                    tmem_st2(col, v[k]);
+                }
+                if (general) {
+                    if (r == 0) {
+                        a0 = v[0];
+                        b0 = v[1];
+                        c0 = v[2];
+                        t00 = t11 = 1.0;
+                        t01 = t10 = 0.0;
+                    } else {
+                        const double cp = __ldcg(out + 2 * NB + gl * R + r - 1), e = v[0] * cp;
+                        const double n00 = fma(v[1], t00, -(e * t10)), n01 = fma(v[1], t01, -(e * t11));
+                        const double sc = pow2_norm(n00, n01);
+                        t10 = t00 * sc;
+                        t11 = t01 * sc;
+                        t00 = n00 * sc;
+                        t01 = n01 * sc;
+                    }
+                    e1 = gl > 0 ? __ldcg(out + 2 * NB + gl * R - 1) : 0.0;
+                }
                 __syncwarp();
             }
         }
-        unsigned next = 0;
-        if (lane == 0) next = atomicAdd(P.work + S, 1u);
-        tl = stride + (int)__shfl_sync(kFull, next, 0);
+        (void)c0;
+        const double c_in = gl > 0 ? e1 : 0.0;
+        tmem_wait_st();
+        if (ROWS) {
+#pragma unroll
+            for (int kk = 0; kk < R / 4; kk++) {
+                unsigned u[3][8];
+#pragma unroll
+                for (int k = 0; k < 3; k++) tmem_ld8(tm + kk * 24 + 8 * k, u[k]);
+                tmem_wait8(u[0]);
+                tmem_after8(u[1]);
+                tmem_after8(u[2]);
+                if (on) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        const double v[4] = {pk_get(u[k], 0), pk_get(u[k], 1), pk_get(u[k], 2), pk_get(u[k], 3)};
+                        st4_cg(out + k * NB + gl * R + 4 * kk, v);
+                    }
+                }
+                __syncwarp();
+            }
+        } else {
+            // the first row's matrix, the scan, then pivot_rows' second pass
+            {
+                const double e = a0 * c_in;
+                const double n00 = fma(t00, b0, t01), n10 = fma(t10, b0, t11);
+                t01 = -(t00 * e);
+                t11 = -(t10 * e);
+                t00 = n00;
+                t10 = n10;
+                const double sc = pow2_norm(t00, t01);
+                t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
+            }
+            unsigned u[3][8];
+#pragma unroll
+            for (int k = 0; k < 3; k++) tmem_ld8(tm + 8 * k, u[k]);
+            double th, thp, cp = c_in;
+            continuant_scan<G>(t00, t01, t10, t11, gl, th, thp);
+            bool bad = false;
+#pragma unroll
+            for (int kk = 0; kk < R / 4; kk++) {
+                tmem_wait8(u[0]);
+                tmem_after8(u[1]);
+                tmem_after8(u[2]);
+                double vi[4], vh[4], vq[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    vh[i] = pk_get(u[0], i);
+                    vi[i] = pk_get(u[1], i);
+                    vq[i] = pk_get(u[2], i);
+                }
+                if (kk < R / 4 - 1) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) tmem_ld8(tm + (kk + 1) * 24 + 8 * k, u[k]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const double n = fma(vi[i], th, -(vh[i] * cp * thp));
+                    bad |= continuant_singular(n, th);
+                    vi[i] = th * rcp_nr(n);
+                    cp = vq[i];
+                    vh[i] *= vi[i];
+                    vq[i] *= vi[i];
+                    thp = th;
+                    th = n;
+                }
+                if (kk == 1) {
+                    const double sc = pow2_norm(th, thp);
+                    th *= sc;
+                    thp *= sc;
+                }
+                if (on) {
+                    st4_cg(out + gl * R + 4 * kk, vi);
+                    st4_cg(out + NB + gl * R + 4 * kk, vh);
+                    st4_cg(out + 2 * NB + gl * R + 4 * kk, vq);
+                }
+                __syncwarp();
+            }
+            if (on && bad) err |= kErrSingular;
+        }
+        if (err) atomicOr(a.err, err);
+        __syncwarp();
     }
+    __syncthreads();
+    if (w == 0) tmem_free<kFacColumns>(tmem_base);
 }
 
 // The factored rows of one segment as a lane holds them for its sub-steps,
@@ -1489,67 +1701,11 @@ __global__ void __launch_bounds__(WPB * 32,
 // 5.2 ms; 30,011 with 11 to 500 sub-steps 0.60 -> 0.25 ms; 64 tracers 152 ->
 // 131 us.  FP64 pipe 52 % (its operand reads ~70 %), stalls per issue:
 // dependent FP64 1.9, shuffles and tensor memory 0.7 to 1.2.
-constexpr int kPkRows = 16;
-constexpr int kPkLanes = NB / kPkRows;    // lanes per tracer
-constexpr int kPkTracers = 32 / kPkLanes; // tracers per warp
 constexpr int kPkWarps = 4;               // one per TMEM lane quarter
 constexpr int kPkColumns = 128;           // TMEM columns of a block: 3 blocks per SM hold 384 of 512
 
 __device__ __forceinline__ double pk_up(double v, int d) { return __shfl_up_sync(kFull, v, d, kPkLanes); }
 __device__ __forceinline__ double pk_down(double v, int d) { return __shfl_down_sync(kFull, v, d, kPkLanes); }
-
-// Sixteen (eight) 32-bit TMEM columns of the warp's lanes.  The loads are
-// asynchronous: the registers are valid after tmem_wait, which names them so
-// that no use is scheduled before it (tmem_after8: a further load that the same
-// wait covers).
-struct Tmem16 {
-    unsigned r[16];
-    __device__ __forceinline__ double d(int i) const { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
-};
-__device__ __forceinline__ void tmem_ld16(unsigned t, Tmem16 &u)
-{
-    unsigned *r = u.r;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(t));
-}
-__device__ __forceinline__ void tmem_ld8(unsigned t, unsigned *r)
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(t));
-}
-__device__ __forceinline__ void tmem_wait(Tmem16 &u)
-{
-    unsigned *r = u.r;
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
-}
-__device__ __forceinline__ void tmem_after8(unsigned *r)
-{
-    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
-}
-__device__ __forceinline__ void tmem_wait8(unsigned *r)
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
-}
-__device__ __forceinline__ void tmem_st8(unsigned t, const unsigned *r)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t), "r"(r[0]), "r"(r[1]),
-                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-
-__device__ __forceinline__ void pk_set(unsigned *r, int i, double v)
-{
-    r[2 * i] = (unsigned)__double2loint(v);
-    r[2 * i + 1] = (unsigned)__double2hiint(v);
-}
-__device__ __forceinline__ double pk_get(const unsigned *r, int i) { return __hiloint2double((int)r[2 * i + 1], (int)r[2 * i]); }
 
 // TMEM columns of the four rows of chunk k: their (g, 1/d) pairs, their E,
 // their dt src/d.
@@ -1639,10 +1795,7 @@ __global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams
     volatile PkWalk &walk = walk_smem;
     const int me = threadIdx.x, w = me >> 5, gl = me & (kPkLanes - 1);
     if (w == 0) {
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(&tmem_base);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "n"(kPkColumns)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        tmem_alloc<kPkColumns>(&tmem_base);
     }
     __syncthreads();
     const unsigned tm = tmem_base + ((unsigned)(w * 32) << 16);   // the warp's lane quarter
@@ -1830,7 +1983,7 @@ __global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams
                 }
                 tmem_st8(pk_fwd(tm, r2 / 2) + 8 * (r2 & 1), u);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tmem_wait_st();
 #pragma unroll
             for (int lv = 0; (1 << lv) < kPkLanes; lv++) {
                 const int off = 1 << lv;
@@ -1957,8 +2110,7 @@ __global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams
         for (int r = 0; r < R; r += 4) st4(row + r, N + r);
     }
     __syncthreads();
-    if (w == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kPkColumns));
+    if (w == 0) tmem_free<kPkColumns>(tmem_base);
 }
 
 template <int S, bool SRC>
@@ -2123,7 +2275,7 @@ __global__ void __launch_bounds__(kWarps * 32, (NB <= 256 ? 20 : 12)) plain_step
         load_rows(fac_ptr(P, S, 0, set, tl), lane, F.h, F.inv, F.q);
 #pragma unroll
         for (int r = 0; r < kR; r += 4) ld4(Nrow + r, N + r);
-        const unsigned err = pivot_rows(F.h, F.inv, F.q, lane);
+        const unsigned err = pivot_rows<kR, 32>(F.h, F.inv, F.q, lane);
         if (__any_sync(kFull, err != 0)) {
             if (lane == 0) atomicOr(a.err, kErrSingular);
             return;
@@ -2154,7 +2306,7 @@ __global__ void __launch_bounds__(256) seg_pre_kernel(FusedParams P)
         if (g.active) {
             const Bg bg = load_bg(a, t, g);
             const int dis = a.dis ? a.dis[t] : 0;
-            const SegTerms<0> T = seg_terms<0>(P.gt, bg, dis, a, g, t, P.ic_stride);
+            const SegTerms T = seg_terms(bg, dis, g);
             const DppForm on = dpp_form(P.mp, P.mp.dpp_model, bg, segment_tacc(P.mp, a, g));
             o.n_gas = T.n_gas;
             o.kbt = T.kbt;
@@ -2351,30 +2503,22 @@ cudaError_t launch_secondary(Context &ctx, const FusedParams &P)
 template <int S, bool ROWS>
 cudaError_t launch_factor(Context &ctx, const FusedParams &P)
 {
-    constexpr size_t smem = (size_t)kTab * kTabStride * sizeof(double) + kFacWarps * sizeof(WarpSmem);
-    // blocks per SM, per instantiation: found once (thread-safe static initialisation)
-    struct Occupancy { cudaError_t e; int resident; };
-    static const Occupancy occ = [] {
-        Occupancy o{cudaSuccess, 0};
-        o.e = cudaFuncSetAttribute(factor_kernel<S, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem);
-        if (o.e == cudaSuccess)
-            o.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.resident, factor_kernel<S, ROWS>,
-                                                                kFacWarps * 32, smem);
-        return o;
-    }();
-    if (occ.e != cudaSuccess) return occ.e;
-    if (occ.resident < 1) return cudaErrorInvalidConfiguration;
-    const int resident = occ.resident;
+    constexpr size_t smem = (size_t)kFacTabs * NB * sizeof(double2) + (S == 0 ? kFacWarps * kCoulWarp : 0) * sizeof(double);
+    static_assert(2 * (smem + 8192) <= 227 * 1024, "two blocks per SM");
+    static const cudaError_t attr = cudaFuncSetAttribute(factor_kernel<S, ROWS>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess) return attr;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    long long blocks = ((long long)P.nt + kFacWarps - 1) / kFacWarps;
-    const long long full = (long long)nsm * resident;
+    const long long systems = (long long)P.nt * (P.g1 - P.g0) * P.sets;
+    if (systems > 0x7fff0000LL) return cudaErrorInvalidValue;
+    long long blocks = (systems + kFacWarps * kPkTracers - 1) / (kFacWarps * kPkTracers);
+    // the occupancy query counts one block per SM for any kernel that allocates
+    // TMEM; kFacBlocks of these fit by registers, columns and shared memory
+    const long long full = (long long)nsm * kFacBlocks;
     if (blocks > full) blocks = full;
     if (blocks < 1) return cudaSuccess;
-    const cudaError_t ez = cudaMemsetAsync(P.work + S, 0, sizeof(unsigned), ctx.stream);
-    if (ez != cudaSuccess) return ez;
     factor_kernel<S, ROWS><<<(unsigned)blocks, kFacWarps * 32, smem, ctx.stream>>>(P);
     return cudaGetLastError();
 }
@@ -2621,11 +2765,9 @@ int fused_reserve(Context &ctx, int cap)
     dev_free(ctx, ctx.d_fac);
     dev_free(ctx, ctx.d_np_seg);
     dev_free(ctx, ctx.d_segpre);
-    dev_free(ctx, ctx.d_work);
     dev_free(ctx, ctx.d_order);
     ctx.d_inje = ctx.d_eta_scale = ctx.d_fac = ctx.d_np_seg = nullptr;
     ctx.d_segpre = nullptr;
-    ctx.d_work = nullptr;
     ctx.d_order = nullptr;
     ctx.fused_chunk = ctx.fused_nseg = ctx.fused_sets = 0;
     const size_t rows = (size_t)nseg * chunk * NB;
@@ -2634,7 +2776,6 @@ int fused_reserve(Context &ctx, int cap)
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_inje, rows * sizeof(double)));
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_eta_scale, (size_t)cap * sizeof(double)));
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_segpre, (size_t)nseg * chunk * sizeof(SegPre)));
-    CROMA_CUDA(dev_alloc(ctx, &ctx.d_work, 2 * sizeof(unsigned)));
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_order, (2 * kOrderBins + (size_t)chunk) * sizeof(int)));
     ctx.fused_chunk = (int)chunk;
     ctx.fused_nseg = nseg;
@@ -2766,7 +2907,6 @@ static int fused_chunks(Context &ctx, FusedParams &P, int nslots, bool perstep)
     P.sets = ctx.fused_sets;
     P.fac = ctx.d_fac;
     P.pre = static_cast<SegPre *>(ctx.d_segpre);
-    P.work = ctx.d_work;
     // chunks: the workspace's uniform split, or the host pipeline's bounds
     // (each within the workspace chunk), whose uploads gate the chunk and
     // whose downloads follow it
