@@ -235,6 +235,9 @@ void croma_b200_destroy(CromaB200Context *h)
     for (auto e : c.pipe_done) cudaEventDestroy(e);
     for (auto e : c.pipe_done_p) cudaEventDestroy(e);
     if (c.pipe_start) cudaEventDestroy(c.pipe_start);
+    if (c.side_begin) cudaEventDestroy(c.side_begin);
+    if (c.side_end) cudaEventDestroy(c.side_end);
+    if (c.side_stream) cudaStreamDestroy(c.side_stream);
     if (c.h2d_stream) cudaStreamDestroy(c.h2d_stream);
     if (c.d2h_stream) cudaStreamDestroy(c.d2h_stream);
     if (c.stream) cudaStreamDestroy(c.stream);
@@ -434,9 +437,9 @@ int snapshot_impl(Context &c, const CromaB200Snapshot *s, int sync)
     a.sched = c.sched;
     a.err = c.d_err;
     int rc = run_schedule(c, a);
-    if (rc) return rc;
-    rc = run_fused(c, a);   // both paths; the plain one runs its per-step kernels
-    if (rc) return rc;
+    if (!rc) rc = run_fused(c, a);   // both paths; the plain one runs its per-step kernels
+    const int rj = join_schedule(c);
+    if (rc || rj) return rc ? rc : rj;
     if (sync) return check_err(c);
     return 0;
 }
@@ -736,6 +739,11 @@ int croma_b200_set_priority(CromaB200Context *h, int priority)
     CROMA_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
     cudaStreamDestroy(c.stream);
     c.stream = s;
+    if (c.side_stream) {   // idle: every snapshot's last kernels wait for it
+        cudaStreamDestroy(c.side_stream);
+        c.side_stream = nullptr;
+        CROMA_CUDA(cudaStreamCreateWithPriority(&c.side_stream, cudaStreamNonBlocking, priority));
+    }
     return 0;
 }
 

@@ -135,6 +135,10 @@ struct Context {
     unsigned long long *d_keys = nullptr, *d_keys_alt = nullptr;
     int *d_vals = nullptr, *d_vals_alt = nullptr, *d_seg_aux = nullptr;
 
+    cudaStream_t side_stream = nullptr;   // bucket build
+    cudaEvent_t side_begin = nullptr, side_end = nullptr;
+    int side_open = 0;                // work on it that the context stream has not waited for
+
     double *d_inje = nullptr;         // electron source per segment (fused workspace)
     double *d_eta_scale = nullptr;    // [cap] Dpp eta-cap scale of the current slot
 
@@ -221,7 +225,11 @@ void free_ic_stage(Context &ctx);
 int ic_rows(Context &ctx, double z, double *d_out);
 // schedule.cu
 int schedule_reserve(Context &ctx, int cap);
+// sub-step counts on the context stream, buckets on the side stream beside
+// what follows; join_schedule makes the context stream wait for them (every
+// run_schedule is followed by one, whatever fails between)
 int run_schedule(Context &ctx, const SnapArgs &a);
+int join_schedule(Context &ctx);
 // fused.cu: both paths (the plain one as per-step kernels, one slot at a time)
 int fused_reserve(Context &ctx, int cap);
 // device bytes fused_reserve allocates for cap tracers under a workspace cap

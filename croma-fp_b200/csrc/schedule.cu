@@ -128,7 +128,8 @@ __global__ void make_keys_kernel(int n, const int *nsub, const int *non, unsigne
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    keys[t] = ((unsigned long long)(unsigned)nsub[t] << 32) | (unsigned)non[t];
+    // both at most 1e6: 20 bits each
+    keys[t] = ((unsigned long long)(unsigned)nsub[t] << 20) | (unsigned)non[t];
     vals[t] = t;
 }
 
@@ -165,13 +166,150 @@ __global__ void seg_rank_kernel(int n, const int *nseg_dev, const int *seg_by_fi
 }
 
 __global__ void assign_bucket_kernel(int n, const int *seg_incl, const int *sorted_t,
-                                     const int *bucket_of_seg, int *bucket_ids, int *bucket_count)
+                                     const int *bucket_of_seg, int *bucket_ids)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int b = bucket_of_seg[seg_incl[i] - 1];
     bucket_ids[sorted_t[i]] = b;
-    atomicAdd(&bucket_count[b], 1);
+}
+
+// The same for a run of at most kBucketOneBlock tracers, by one block: the
+// distinct keys in a hash table in shared memory (one insertion per key and
+// warp), each with its first tracer; a bucket's number is the count of first
+// tracers before its own; the members are placed in tracer order by one warp.
+// Three radix sorts and their dozen small kernels took 30 us of GPU time and
+// some 25 launches at 64 tracers, 33 us at 999; this takes 3.7 and 7.3 us and
+// one.  Above that the block's table outgrows its shared memory.
+constexpr int kBucketOneBlock = 4096;
+constexpr int kBucketThreads = 1024;
+
+__host__ __device__ __forceinline__ int bucket_table(int n)   // a power of two, at least 2 n
+{
+    int h = 64;
+    while (h < 2 * n) h <<= 1;
+    return h;
+}
+
+size_t bucket_smem(int n)   // keys and first tracers of the table, slots of the tracers
+{
+    return (size_t)bucket_table(n) * (sizeof(unsigned long long) + sizeof(int)) + (size_t)n * sizeof(int);
+}
+
+// exclusive prefix sum of v over the block, and its total
+__device__ __forceinline__ int block_prefix(int v, int *warp_sums, int &total)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int s = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, s, off);
+        if (lane >= off) s += o;
+    }
+    if (lane == 31) warp_sums[w] = s;
+    __syncthreads();
+    if (w == 0) {
+        const int ws = warp_sums[lane];
+        int x = ws;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, x, off);
+            if (lane >= off) x += o;
+        }
+        warp_sums[lane] = x - ws;
+        if (lane == 31) warp_sums[32] = x;
+    }
+    __syncthreads();
+    const int before = warp_sums[w] + s - v;
+    total = warp_sums[32];
+    __syncthreads();
+    return before;
+}
+
+__global__ void __launch_bounds__(kBucketThreads) bucket_small_kernel(int n, const int *nsub, const int *non,
+                                                                      int *bucket_ids, int *bucket_indices, int *nbuckets)
+{
+    extern __shared__ unsigned long long bk_smem[];
+    __shared__ int warp_sums[33];
+    constexpr unsigned long long kEmpty = ~0ull;
+    const int H = bucket_table(n), lane = threadIdx.x & 31;
+    unsigned long long *keys = bk_smem;                  // [H]
+    int *first = reinterpret_cast<int *>(keys + H);      // [H] first tracer of the slot's key
+    int *slot = first + H;                               // [n] slot of each tracer
+    int *id = reinterpret_cast<int *>(keys);             // [H] bucket of each slot, once the keys are done
+    int *start = id + H;                                 // [n] next place of each bucket (2 H ints in keys, H >= 2 n)
+    const int top = (n + 31) & ~31;
+    for (int h = threadIdx.x; h < H; h += blockDim.x) {
+        keys[h] = kEmpty;
+        first[h] = 0x7fffffff;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < top; t += blockDim.x) {
+        const bool on = t < n;
+        const unsigned long long key = on ? ((unsigned long long)(unsigned)nsub[t] << 32) | (unsigned)non[t] : kEmpty;
+        const unsigned peers = __match_any_sync(0xffffffffu, key);
+        const int leader = __ffs(peers) - 1;
+        int h = 0;
+        if (on && lane == leader) {
+            h = (int)((key * 0x9e3779b97f4a7c15ull) >> 40) & (H - 1);
+            for (int probe = 0; probe < H; probe++, h = (h + 1) & (H - 1)) {   // a free slot is always met
+                unsigned long long at = *(volatile unsigned long long *)(keys + h);
+                if (at == kEmpty) at = atomicCAS(keys + h, kEmpty, key);
+                if (at == kEmpty || at == key) break;
+            }
+            atomicMin(first + h, t);   // the lowest lane of the warp's equals
+        }
+        h = __shfl_sync(0xffffffffu, h, leader);
+        if (on) slot[t] = h;
+    }
+    __syncthreads();
+    // bucket numbers in the order of the first tracers
+    int total = 0;
+    for (int t0 = 0; t0 < n; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x;
+        const bool lead = t < n && first[slot[t]] == t;
+        int here;
+        const int before = block_prefix(lead ? 1 : 0, warp_sums, here);
+        if (lead) id[slot[t]] = total + before;
+        total += here;
+    }
+    if (threadIdx.x == 0) *nbuckets = total;
+    for (int b = threadIdx.x; b < n; b += blockDim.x) start[b] = 0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < top; t += blockDim.x) {
+        const bool on = t < n;
+        const int b = on ? id[slot[t]] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, b);
+        if (on) {
+            bucket_ids[t] = b;
+            slot[t] = b;
+            if (lane == __ffs(peers) - 1) atomicAdd(start + b, __popc(peers));
+        }
+    }
+    __syncthreads();
+    int base = 0;
+    for (int b0 = 0; b0 < total; b0 += blockDim.x) {
+        const int b = b0 + threadIdx.x, c = b < total ? start[b] : 0;
+        int here;
+        const int before = block_prefix(c, warp_sums, here);
+        if (b < total) start[b] = base + before;
+        base += here;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        for (int t = lane; t < top; t += 32) {
+            const bool on = t < n;
+            const int b = on ? slot[t] : -1;
+            const unsigned peers = __match_any_sync(0xffffffffu, b);
+            const int at = on ? start[b] : 0;
+            __syncwarp();
+            if (on) {
+                bucket_indices[at + __popc(peers & ((1u << lane) - 1u))] = t;
+                if (lane == __ffs(peers) - 1) start[b] = at + __popc(peers);
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // Members listed bucket by bucket in ascending tracer order: a stable
@@ -210,10 +348,10 @@ int schedule_reserve(Context &ctx, int cap)
     ctx.sched.bucket_indices = p + 5 * n;
     ctx.sched.nbuckets = p + 6 * n;
     ctx.sched.capped = ctx.d_capped;
-    // keys/vals double buffers + aux (head/scan, first keys, seg ids, bucket_of_seg, counts)
+    // keys/vals double buffers + aux (head/scan, first segments, bucket_of_seg, segments by first tracer)
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_keys, n * 3 * sizeof(unsigned long long)));
     ctx.d_keys_alt = ctx.d_keys + n;
-    CROMA_CUDA(dev_alloc(ctx, &ctx.d_vals, n * 8 * sizeof(int)));
+    CROMA_CUDA(dev_alloc(ctx, &ctx.d_vals, n * 6 * sizeof(int)));
     ctx.d_vals_alt = ctx.d_vals + n;
     ctx.d_seg_aux = ctx.d_vals + 2 * n;
     size_t b1 = 0, b2 = 0;
@@ -223,56 +361,70 @@ int schedule_reserve(Context &ctx, int cap)
     CROMA_CUDA(cub::DeviceScan::InclusiveSum(nullptr, b2, ctx.d_seg_aux, ctx.d_seg_aux, cap, ctx.stream));
     ctx.cub_tmp_bytes = (b1 > b2 ? b1 : b2) + 256;
     CROMA_CUDA(dev_alloc(ctx, &ctx.d_cub_tmp, ctx.cub_tmp_bytes));
+    // above the default 48 KB for runs of more than 1,024 tracers; per device, so here
+    CROMA_CUDA(cudaFuncSetAttribute(bucket_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)bucket_smem(kBucketOneBlock)));
+    if (!ctx.side_stream) {   // of the context stream's priority: the snapshot ends with it
+        int priority = 0;
+        CROMA_CUDA(cudaStreamGetPriority(ctx.stream, &priority));
+        CROMA_CUDA(cudaStreamCreateWithPriority(&ctx.side_stream, cudaStreamNonBlocking, priority));
+    }
+    if (!ctx.side_begin) CROMA_CUDA(cudaEventCreateWithFlags(&ctx.side_begin, cudaEventDisableTiming));
+    if (!ctx.side_end) CROMA_CUDA(cudaEventCreateWithFlags(&ctx.side_end, cudaEventDisableTiming));
     return 0;
 }
 
-int run_schedule(Context &ctx, const SnapArgs &a)
+// Buckets are for the caller (get_schedule); nothing of the snapshot reads
+// them.  So they are built on a stream of their own from the sub-step counts
+// on, beside the snapshot's kernels, which wait on FP64 latency most of the
+// time.  A snapshot of 64 tracers: 118 to 98 us; GPU time of one of 999 629 to
+// 579 us, of 30,011 814 to 741 us, the bucket kernels overlapping the rest.
+static int run_buckets(Context &ctx, const SnapArgs &a, cudaStream_t st)
 {
     const int n = a.ntracer;
+    if (n <= kBucketOneBlock) {
+        bucket_small_kernel<<<1, kBucketThreads, bucket_smem(n), st>>>(n, a.sched.nsub, a.sched.non, a.sched.bucket_ids,
+                                                             a.sched.bucket_indices, a.sched.nbuckets);
+        CROMA_CUDA(cudaGetLastError());
+        ctx.last_launches += 1;
+        return 0;
+    }
     const int blk = 256, grd = (n + blk - 1) / blk;
-    nsub_kernel<<<grd, blk, 0, ctx.stream>>>(ctx.mp, n, a.bg_curr, a.ic_curr, ctx.h_p[0][0],
-                                             ctx.h_p[0][NB - 1], ctx.h_p[1][0], ctx.h_p[1][NB - 1],
-                                             a.dt_snap, a.allow_interp, a.sched);
-    CROMA_CUDA(cudaGetLastError());
-    ctx.last_launches += 1;
-
-    // ---- bucket build ----
+    int bits = 1;   // all ones in them is no tracer's index
+    while ((1LL << bits) - 1 < n) bits++;
     const size_t N = (size_t)n;
     int *head = ctx.d_seg_aux;              // [n] head flags, scanned in place
     int *first_seg = ctx.d_seg_aux + N;     // [n]
     int *bucket_of_seg = ctx.d_seg_aux + 2 * N;
     int *seg_by_first = ctx.d_seg_aux + 3 * N;
-    int *counts = ctx.d_seg_aux + 4 * N;
     unsigned long long *first_keys = ctx.d_keys + 2 * N;
     size_t tmp = ctx.cub_tmp_bytes;
 
-    make_keys_kernel<<<grd, blk, 0, ctx.stream>>>(n, a.sched.nsub, a.sched.non, ctx.d_keys, ctx.d_vals);
+    make_keys_kernel<<<grd, blk, 0, st>>>(n, a.sched.nsub, a.sched.non, ctx.d_keys, ctx.d_vals);
     cub::DoubleBuffer<unsigned long long> kb(ctx.d_keys, ctx.d_keys_alt);
     cub::DoubleBuffer<int> vb(ctx.d_vals, ctx.d_vals_alt);
-    CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, kb, vb, n, 0, 64, ctx.stream));
+    CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, kb, vb, n, 0, 40, st));
     const unsigned long long *skeys = kb.Current();
     const int *sorted_t = vb.Current();
-    seg_heads_kernel<<<grd, blk, 0, ctx.stream>>>(n, skeys, head);
+    seg_heads_kernel<<<grd, blk, 0, st>>>(n, skeys, head);
     tmp = ctx.cub_tmp_bytes;
-    CROMA_CUDA(cub::DeviceScan::InclusiveSum(ctx.d_cub_tmp, tmp, head, head, n, ctx.stream));
+    CROMA_CUDA(cub::DeviceScan::InclusiveSum(ctx.d_cub_tmp, tmp, head, head, n, st));
     // sorted_t lives in one of the two value buffers; keep it intact while the
     // segment-first pairs are sorted through the other key buffer and aux ints.
     // (first tracer, segment) pairs; unused tail entries carry all-ones keys
     // so that they sort last.
-    CROMA_CUDA(cudaMemsetAsync(first_keys, 0xFF, N * sizeof(unsigned long long), ctx.stream));
-    seg_first_kernel<<<grd, blk, 0, ctx.stream>>>(n, head, sorted_t, first_keys, first_seg);
+    CROMA_CUDA(cudaMemsetAsync(first_keys, 0xFF, N * sizeof(unsigned long long), st));
+    seg_first_kernel<<<grd, blk, 0, st>>>(n, head, sorted_t, first_keys, first_seg);
     {
         unsigned long long *fk_alt = (kb.Current() == ctx.d_keys) ? ctx.d_keys_alt : ctx.d_keys;
         cub::DoubleBuffer<unsigned long long> fkb(first_keys, fk_alt);
         cub::DoubleBuffer<int> fvb(first_seg, seg_by_first);
         tmp = ctx.cub_tmp_bytes;
-        CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, fkb, fvb, n, 0, 32, ctx.stream));
-        seg_rank_kernel<<<grd, blk, 0, ctx.stream>>>(n, head + (n - 1), fvb.Current(), bucket_of_seg);
-        CROMA_CUDA(cudaMemsetAsync(counts, 0, N * sizeof(int), ctx.stream));
-        assign_bucket_kernel<<<grd, blk, 0, ctx.stream>>>(n, head, sorted_t, bucket_of_seg,
-                                                          a.sched.bucket_ids, counts);
+        CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, fkb, fvb, n, 0, bits, st));
+        seg_rank_kernel<<<grd, blk, 0, st>>>(n, head + (n - 1), fvb.Current(), bucket_of_seg);
+        assign_bucket_kernel<<<grd, blk, 0, st>>>(n, head, sorted_t, bucket_of_seg, a.sched.bucket_ids);
         CROMA_CUDA(cudaMemcpyAsync(a.sched.nbuckets, head + (n - 1), sizeof(int),
-                                   cudaMemcpyDeviceToDevice, ctx.stream));
+                                   cudaMemcpyDeviceToDevice, st));
     }
     CROMA_CUDA(cudaGetLastError());
     ctx.last_launches += 6;
@@ -281,16 +433,40 @@ int run_schedule(Context &ctx, const SnapArgs &a)
     {
         unsigned long long *k0 = ctx.d_keys, *k1 = ctx.d_keys_alt;
         int *v0 = ctx.d_vals, *v1 = ctx.d_vals_alt;
-        bucket_keys_kernel<<<grd, blk, 0, ctx.stream>>>(n, a.sched.bucket_ids, k0, v0);
+        bucket_keys_kernel<<<grd, blk, 0, st>>>(n, a.sched.bucket_ids, k0, v0);
         cub::DoubleBuffer<unsigned long long> bkb(k0, k1);
         cub::DoubleBuffer<int> bvb(v0, v1);
         tmp = ctx.cub_tmp_bytes;
-        CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, bkb, bvb, n, 0, 32, ctx.stream));
+        CROMA_CUDA(cub::DeviceRadixSort::SortPairs(ctx.d_cub_tmp, tmp, bkb, bvb, n, 0, bits, st));
         CROMA_CUDA(cudaMemcpyAsync(a.sched.bucket_indices, bvb.Current(), N * sizeof(int),
-                                   cudaMemcpyDeviceToDevice, ctx.stream));
+                                   cudaMemcpyDeviceToDevice, st));
     }
     CROMA_CUDA(cudaGetLastError());
     ctx.last_launches += 6;
+    return 0;
+}
+
+int run_schedule(Context &ctx, const SnapArgs &a)
+{
+    const int n = a.ntracer;
+    nsub_kernel<<<(n + 255) / 256, 256, 0, ctx.stream>>>(ctx.mp, n, a.bg_curr, a.ic_curr, ctx.h_p[0][0],
+                                                         ctx.h_p[0][NB - 1], ctx.h_p[1][0], ctx.h_p[1][NB - 1],
+                                                         a.dt_snap, a.allow_interp, a.sched);
+    CROMA_CUDA(cudaGetLastError());
+    ctx.last_launches += 1;
+    CROMA_CUDA(cudaEventRecord(ctx.side_begin, ctx.stream));
+    CROMA_CUDA(cudaStreamWaitEvent(ctx.side_stream, ctx.side_begin, 0));
+    const int rc = run_buckets(ctx, a, ctx.side_stream);
+    CROMA_CUDA(cudaEventRecord(ctx.side_end, ctx.side_stream));
+    ctx.side_open = 1;
+    return rc;
+}
+
+int join_schedule(Context &ctx)
+{
+    if (!ctx.side_open) return 0;
+    ctx.side_open = 0;
+    CROMA_CUDA(cudaStreamWaitEvent(ctx.stream, ctx.side_end, 0));
     return 0;
 }
 
