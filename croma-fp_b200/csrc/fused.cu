@@ -569,22 +569,25 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
     }
     // rows a, b, c of chunk k (four rows) of the warp's lanes: 8 columns each
     const unsigned tm = tmem_base + ((unsigned)((w & 3) * 32) << 16) + (w >> 2) * 128;
-    // A unit: kPkTracers (segment, set) pairs of one tracer, or, with fewer pairs
-    // than that, those of several tracers; unit numbers run over the tracers
-    // first, so that pairs beyond a tracer's last segment fall evenly on the warps.
-    const int per = (P.g1 - P.g0) * P.sets, pairs = min(per, kPkTracers), tracers = kPkTracers / pairs;
-    const int nq = (P.nt + tracers - 1) / tracers;
-    const int units = (per + pairs - 1) / pairs * nq, stride = gridDim.x * kFacWarps;
-    const int sub = (lane / G) / pairs, off = (lane / G) - sub * pairs;   // the group's place in the unit
+    // A unit: kPkTracers segments of one tracer and one set, or, with fewer
+    // segments than that, those of several tracers; unit numbers run over the
+    // tracers first, so that segments beyond a tracer's last fall evenly on the
+    // warps, and over the sets last: most windowed segments need one of the two,
+    // and a warp whose systems all need none of its set leaves at once (28 to
+    // 25 us a slot at 10,000 windowed tracers).
+    const int nslot = P.g1 - P.g0, segs = min(nslot, kPkTracers), tracers = kPkTracers / segs;
+    const int nq = (P.nt + tracers - 1) / tracers, nblk = (nslot + segs - 1) / segs;
+    const int units = nblk * nq * P.sets, stride = gridDim.x * kFacWarps;
+    const int sub = (lane / G) / segs, off = (lane / G) - sub * segs;   // the group's place in the unit
     double *coul = reinterpret_cast<double *>(tab + kFacTabs * NB) + w * kCoulWarp;
     const double2 *row = tab + gl;                // table k, row r of the lane: row[k * NB + r * G]
     const int group = w * kPkTracers + lane / G;
     auto locate = [&](int unit, int &tl, int &gi, int &set) {
-        const int blk = unit / nq, slot = blk * pairs + off;
-        tl = (unit - blk * nq) * tracers + sub;
-        gi = slot / P.sets;
-        set = slot - gi * P.sets;
-        return unit < units && sub < tracers && tl < P.nt && slot < per;
+        const int b = unit / nq;
+        set = b / nblk;
+        gi = (b - set * nblk) * segs + off;
+        tl = (unit - b * nq) * tracers + sub;
+        return unit < units && sub < tracers && tl < P.nt && gi < nslot;
     };
     auto fetch = [&](int unit, int buf) {         // the unit's scalars, 16 bytes a lane
         int tl, gi, set;
@@ -2303,7 +2306,12 @@ __global__ void __launch_bounds__(256) seg_pre_kernel(FusedParams P)
         const int t = P.t0 + tl;
         SegPre o{};
         const SegInfo g = segment_of(P, t, P.g0 + gi);
-        if (g.active) {
+        if (!g.active) {   // nothing reads more of it than its flags; 112 strided bytes a
+                           // thread bound this kernel (43 to 27 us, most of 16 slots inactive)
+            *reinterpret_cast<int4 *>(&P.pre[i].flags) = make_int4(0, 0, 0, 0);
+            continue;
+        }
+        {
             const Bg bg = load_bg(a, t, g);
             const int dis = a.dis ? a.dis[t] : 0;
             const SegTerms T = seg_terms(bg, dis, g);
@@ -2799,11 +2807,23 @@ static int pipe_download(Context &ctx, const FusedParams &P, cudaEvent_t ev, dou
     return 0;
 }
 
+static void launch_seg_pre(Context &ctx, const FusedParams &P)
+{
+    const long long total = (long long)(P.g1 - P.g0) * P.nt;
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    long long blocks = (total + 255) / 256;
+    if (blocks > 8LL * nsm) blocks = 8LL * nsm;
+    seg_pre_kernel<<<(unsigned)blocks, 256, 0, ctx.stream>>>(P);
+}
+
 // pk >= 0 (host pipeline, all segments in one launch): the chunk's upload is
 // awaited only before the first steps kernel -- the per-segment scalars and
 // the factored rows do not read the spectra -- and the proton rows go back as
-// soon as the proton steps are done.
-static int fused_range(Context &ctx, FusedParams &P, int g0, int g1, bool perstep, int pk = -1)
+// soon as the proton steps are done.  scalars_done: the slots' scalars are
+// there already, P.pre at this slot's.
+static int fused_range(Context &ctx, FusedParams &P, int g0, int g1, bool perstep, int pk = -1, bool scalars_done = false)
 {
     const SnapArgs &a = P.a;
     const int protons = ctx.mp.species_mask & CROMA_SPECIES_PROTON;
@@ -2828,14 +2848,8 @@ static int fused_range(Context &ctx, FusedParams &P, int g0, int g1, bool perste
         ctx.last_launches += 1;
         P.eta_scale = ctx.d_eta_scale;
     }
-    if (protons || electrons) {
-        const long long total = (long long)(g1 - g0) * P.nt;
-        int dev = 0, nsm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        long long blocks = (total + 255) / 256;
-        if (blocks > 8LL * nsm) blocks = 8LL * nsm;
-        seg_pre_kernel<<<(unsigned)blocks, 256, 0, ctx.stream>>>(P);
+    if ((protons || electrons) && !scalars_done) {
+        launch_seg_pre(ctx, P);
         ctx.last_launches += 1;
     }
     if (protons) {
@@ -2937,10 +2951,29 @@ static int fused_chunks(Context &ctx, FusedParams &P, int nslots, bool perstep)
             if (rc) return rc;
         } else {
             if (pipe) CROMA_CUDA(cudaStreamWaitEvent(ctx.stream, ctx.pipe_up[k], 0));
-            for (int g = 0; g < nslots; g++) {
-                const int rc = fused_range(ctx, P, g, g + 1, perstep);
-                if (rc) return rc;
+            // one slot per launch; the on-chip path's workspace holds the scalars
+            // of all slots, which do not depend on the spectra, so they take one
+            // launch: 21 us at 16 slots of 10,000 windowed tracers, 16 of 7.3 before
+            const bool once = !perstep && (ctx.mp.species_mask & 3);
+            SegPre *const base = P.pre;
+            if (once) {
+                P.g0 = 0;
+                P.g1 = nslots;
+                cudaEvent_t ev = nullptr;
+                timed_begin(ctx, kKindCoeff, &ev);
+                launch_seg_pre(ctx, P);
+                timed_end(ctx, kKindCoeff, ev);
+                ctx.last_launches += 1;
             }
+            for (int g = 0; g < nslots; g++) {
+                P.pre = once ? base + (size_t)g * P.nt : base;
+                const int rc = fused_range(ctx, P, g, g + 1, perstep, -1, once);
+                if (rc) {
+                    P.pre = base;
+                    return rc;
+                }
+            }
+            P.pre = base;
             if (pipe && pipe->down_p) {
                 const int rc = pipe_download(ctx, P, ctx.pipe_done_p[k], pipe->crp, P.a.crp);
                 if (rc) return rc;
