@@ -1,17 +1,18 @@
 // dsa.cu -- per-snapshot DSA (diffusive shock acceleration) injection into the
-// device-resident tracer spectra, one warp per tracer.
+// device-resident tracer spectra, one block at a time per shocked tracer.
 //
-// For every tracer whose shock fields pass the reference's checks the warp
+// For every tracer whose shock fields pass the reference's checks the block
 //   1. resolves the upstream state (Mach number, temperature, density,
 //      speed; tracer_dsa_resolve_tracer_input, src/tracer_fp_dsa.c:26-108),
 //   2. builds the fresh proton spectrum: efficiency eta(M) (the eight models
 //      of src/DSA_MODELS.c:262-468), slope q = 3r/(r-1), injection momentum
 //      chi p_th, and the normalisation from a 4000-interval Simpson integral of
 //      the kinetic-energy density (src/DSA_MODELS.c:690-776) whose terms are
-//      split over the lanes and combined by a shuffle tree,
+//      split over the block's threads and combined by shuffle trees,
 //   3. builds the suprathermal electron spectrum normalised to the protons at
 //      the proton injection momentum (src/DSA_MODELS.c:1022-1070),
-//   4. optionally computes the reacceleration of the pre-shock spectra
+//   4. optionally computes the reacceleration of the pre-shock spectra, a warp
+//      a species
 //      (positive_delta / drury83 with its eta cap and the adiabatic part,
 //      src/tracer_fp_dsa_reacc.c:60-236): the cumulative momentum integrals
 //      run as warp scans over 32-bin chunks, the energy sums as shuffle trees,
@@ -36,7 +37,18 @@ constexpr double kCCroma = 2.999e10;        // CROMA's c, used by the tracer ene
 constexpr double k4Pi = 12.566370614359172;
 constexpr double kMsunG = 1.99e33;
 constexpr double kPiD = 3.14159265358979323846;
-constexpr int kDsaWarps = 4;
+// Shocks hit a few percent of the tracers, and each costs some 4,000 powers
+// and exponentials.  A block looks at up to kDsaTracers tracers (a thread each)
+// and takes its shocked ones in turn, all threads on one, so that a run's
+// shocks spread over the chip.  FP64 latency bounds it.  Before (a warp per
+// tracer, four in a block that held its shared memory until the last was done:
+// 3 busy warps an SM at 512 bins) and now, 5 % shocked: 131,072 tracers 1.82 ms
+// and 0.58, 1,500 tracers 205 us and 80.  Smaller runs take fewer tracers a
+// block, down to one: eight of 1,500 make some blocks take four shocks in turn
+// (178 us); one of 131,072 costs mostly block launches.
+constexpr int kDsaThreads = 256;
+constexpr int kDsaTracers = 8;
+constexpr int kDsaSpread = 2368;   // blocks, 16 an SM, before a block takes more than one tracer
 
 struct DsaModelCoef {
     int family, reacc;
@@ -60,7 +72,7 @@ struct DsaArgs {
     const double *mach, *prestemp, *presden, *pre_density_cgs, *upstream_speed_cgs, *shock_side_code;
     const double *dsa_trigger, *dsa_mach, *dsa_pre_density, *dsa_flux;
     int has_dsa;
-    int ntracer;
+    int ntracer, per_block;
     double density_unit, dt_gyr;
     int mode, reacc;
     // spectra and sources: element (t, j) at base + t * ts + j * js
@@ -162,18 +174,25 @@ __device__ __forceinline__ double warp_scan(double v, int lane)
     return v;
 }
 
-// 4 pi m_p c^2 x Simpson integral of the energy integrand over [p_inj, p_max]
-__device__ double proton_edens_unit(double pinj, double q, double pmax, int lane)
+// 4 pi m_p c^2 x Simpson integral of the energy integrand over [p_inj, p_max],
+// by the whole block (the arguments are the same in all of its threads)
+__device__ double proton_edens_unit(double pinj, double q, double pmax, double *part)
 {
     if (pinj <= 0.0 || pmax <= 0.0 || pmax <= pinj) return 0.0;
     constexpr int nstep = 4000;
     const double h = (pmax - pinj) / (double)nstep;
     double s = 0.0;
-    for (int i = 1 + lane; i < nstep; i += 32) {
+    for (int i = 1 + threadIdx.x; i < nstep; i += kDsaThreads) {
         const double p = pinj + h * (double)i;
         s += ((i % 2) ? 4.0 : 2.0) * energy_integrand(p, pinj, q, pmax);
     }
     s = warp_sum(s);
+    __syncthreads();   // part's readers of the tracer before are done
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kDsaThreads / 32; w++) s += part[w];
     s += energy_integrand(pinj, pinj, q, pmax) + energy_integrand(pmax, pinj, q, pmax);
     return k4Pi * kMpG * kCExact * kCExact * (s * h / 3.0);
 }
@@ -228,11 +247,38 @@ __device__ bool resolve_input(const DsaArgs &A, int t, double &mach, double &tem
     return true;
 }
 
-// Per-warp shared rows: reacceleration deltas and adiabatic deltas of both
-// species.
+// Reacceleration deltas and adiabatic deltas of both species, the partial sums
+// of the Simpson integral and the species' energy sums.
 struct DsaSmem {
     double dlt[2][NB], ad[2][NB];
+    double part[kDsaThreads / 32];
+    double e_dlt[2], e_ad[2], budget;
 };
+
+// What the injection of one shocked tracer starts from; false: it has none.
+struct DsaShock {
+    double mach, temp, rho1, u1, ratio, u2, q, pmin_p, pmin_e, chi_e, mass_g, vup, vdown;
+};
+__device__ bool dsa_shock(const DsaArgs &A, int t, DsaShock &k)
+{
+    const CromaB200DsaParams &prm = A.prm;
+    if (!resolve_input(A, t, k.mach, k.temp, k.rho1, k.u1)) return false;
+    k.ratio = compression_ratio(k.mach, prm.gamma_gas);
+    if (!(k.ratio > 0.0) || !isfinite(k.ratio)) return false;
+    const double rho2 = k.ratio * k.rho1;
+    k.u2 = k.u1 / k.ratio;
+    k.q = 0.0;
+    if (k.mach > 1.0 && k.ratio > 1.0) k.q = 3.0 * k.ratio / (k.ratio - 1.0);
+    if (!(k.q > 0.0) || !isfinite(k.q)) return false;
+    k.chi_e = (prm.chi_e > 0.0) ? prm.chi_e : prm.chi_p;
+    k.pmin_p = injection_momentum(k.temp, prm.chi_p, kMpG);
+    k.pmin_e = injection_momentum(k.temp, k.chi_e, kMeG);
+    if (!(k.pmin_p > 0.0) || !isfinite(k.pmin_p) || !(k.pmin_e > 0.0) || !isfinite(k.pmin_e)) return false;
+    k.mass_g = A.mass[t] * kMsunG;
+    k.vup = k.mass_g / k.rho1;
+    k.vdown = k.mass_g / rho2;
+    return k.vup > 0.0 && isfinite(k.vup) && k.vdown > 0.0 && isfinite(k.vdown);
+}
 
 // positive_delta (tracer_fp_dsa_reacc.c:60-103): deltas and their energy density
 __device__ double reacc_positive(const DsaArgs &A, int s, const double *N, double vdown, double q,
@@ -339,26 +385,15 @@ __device__ double reacc_adiabatic(const DsaArgs &A, int s, const double *N, doub
     return delta_edens(A, s, ad, pmin, lane);
 }
 
-__global__ void __launch_bounds__(kDsaWarps * 32) dsa_inject_kernel(DsaArgs A)
+// All threads of the block on tracer t.
+__device__ void dsa_tracer(const DsaArgs &A, int t, DsaSmem &sm)
 {
-    extern __shared__ double4 smem_raw[];
-    DsaSmem &sm = reinterpret_cast<DsaSmem *>(smem_raw)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int t = blockIdx.x * kDsaWarps + (threadIdx.x >> 5);
-    if (t >= A.ntracer) return;
     const CromaB200DsaParams &prm = A.prm;
-    double mach, temp, rho1, u1;
-    if (!resolve_input(A, t, mach, temp, rho1, u1)) return;
-    const double ratio = compression_ratio(mach, prm.gamma_gas);
-    if (!(ratio > 0.0) || !isfinite(ratio)) return;
-    const double rho2 = ratio * rho1, u2 = u1 / ratio;
-    double q = 0.0;
-    if (mach > 1.0 && ratio > 1.0) q = 3.0 * ratio / (ratio - 1.0);
-    if (!(q > 0.0) || !isfinite(q)) return;
-    const double chi_e = (prm.chi_e > 0.0) ? prm.chi_e : prm.chi_p;
-    const double pmin_p = injection_momentum(temp, prm.chi_p, kMpG);
-    const double pmin_e = injection_momentum(temp, chi_e, kMeG);
-    if (!(pmin_p > 0.0) || !isfinite(pmin_p) || !(pmin_e > 0.0) || !isfinite(pmin_e)) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    DsaShock k;
+    if (!dsa_shock(A, t, k)) return;   // the same in all threads; true, as the caller found
+    const double mach = k.mach, rho1 = k.rho1, u1 = k.u1, q = k.q, pmin_p = k.pmin_p, pmin_e = k.pmin_e;
+    const double chi_e = k.chi_e, mass_g = k.mass_g, vup = k.vup, vdown = k.vdown;
     const int inj_p = prm.inject_species != 2, inj_e = prm.inject_species != 1;
 
     // fresh protons and electrons
@@ -366,9 +401,9 @@ __global__ void __launch_bounds__(kDsaWarps * 32) dsa_inject_kernel(DsaArgs A)
     const double eta = dsa_eta(mach, prm.eta_model_initial);
     if (mach > 1.0 && prm.gamma_gas > 1.0 && prm.chi_p > 0.0 && prm.pmax_p_mc > 0.0 && eta > 0.0 &&
         pmin_p < prm.pmax_p_mc) {
-        const double unit = proton_edens_unit(pmin_p, q, prm.pmax_p_mc, lane);
-        if (unit > 0.0 && rho1 > 0.0 && u1 > 0.0 && u2 > 0.0)
-            A_p = eta * (0.5 * rho1 * u1 * u1 * u1) / u2 / unit;
+        const double unit = proton_edens_unit(pmin_p, q, prm.pmax_p_mc, sm.part);
+        if (unit > 0.0 && rho1 > 0.0 && u1 > 0.0 && k.u2 > 0.0)
+            A_p = eta * (0.5 * rho1 * u1 * u1 * u1) / k.u2 / unit;
     }
     const bool fresh_p = A_p > 0.0;
     if (fresh_p && inj_e && prm.pmax_e_mc > 0.0 && chi_e > 0.0 && pmin_e < prm.pmax_e_mc && prm.k_ep > 0.0) {
@@ -378,86 +413,93 @@ __global__ void __launch_bounds__(kDsaWarps * 32) dsa_inject_kernel(DsaArgs A)
         if (sp > 0.0 && se > 0.0) A_e = prm.k_ep * (1.0 / (mr * mr * mr)) * A_p * sp / se;
     }
     const bool fresh_e = A_e > 0.0;
-
-    const double mass_g = A.mass[t] * kMsunG;
-    const double vup = mass_g / rho1, vdown = mass_g / rho2;
-    if (!(vup > 0.0) || !isfinite(vup) || !(vdown > 0.0) || !isfinite(vdown)) return;
     const double *Np = A.crp + (size_t)t * A.ts;
     const double *Ne = A.cre + (size_t)t * A.ts;
 
-    // reacceleration deltas of the pre-shock spectra
+    // reacceleration deltas of the pre-shock spectra: warp 0 protons, warp 1 electrons
     double scale = 0.0, energy = 0.0;
     const bool reacc = A.reacc == 1 || A.reacc == 2;
-    if (reacc) {
-        for (int j = lane; j < NB; j += 32) {
-            sm.dlt[0][j] = 0.0;
-            sm.dlt[1][j] = 0.0;
-        }
-        __syncwarp();
-    }
+    if (reacc) __syncthreads();   // the rows' readers of the tracer before are done
     if (A.reacc == 1) {
-        // X_cr = P_cr / P_th with E_cr above xcr_pmin (tracer_dsa_xcr_proton)
-        double e = 0.0;
-        for (int j = lane; j < NB; j += 32)
-            if (A.p[0][j] >= prm.xcr_pmin_pmc) e += ekin_erg(A.p[0][j], 0) * Np[j * A.js] * A.dp[0][j];
-        const double ecr = warp_sum(e) / vdown;
-        const double pth = rho1 * kKbCgs * temp / (prm.mu_mol * kMpG);
-        double xcr = 0.0;
-        if (pth > 0.0 && isfinite(ecr / 3.0) && isfinite(pth) && ecr / 3.0 > 0.0) xcr = (ecr / 3.0) / pth;
-        double eta_int = 0.0;
-        const int ii = prm.eta_model_initial, ir = prm.eta_model_reacc;
-        if (ii >= 0 && ii < 8 && ir >= 0 && ir < 8) {
-            const double ei = dsa_eta(mach, ii), er = dsa_eta(mach, ir);
-            const double x0 = c_models[ir].xcr0;
-            if (x0 <= 0.0) {
-                eta_int = ei;
-            } else {
-                const double wgt = fmin(fmax(xcr / x0, 0.0), 1.0);
-                eta_int = (1.0 - wgt) * ei + wgt * er;
-            }
-        }
-        double extra = eta_int - dsa_eta(mach, ii);
-        if (extra < 0.0 || !isfinite(extra)) extra = 0.0;
-        const double budget = extra * 0.5 * mass_g * u1 * u1;
-        if (budget > 0.0) {
-            const double ep = reacc_positive(A, 0, Np, vdown, q, pmin_p, sm.dlt[0], lane);
-            const double ee = reacc_positive(A, 1, Ne, vdown, q, pmin_e, sm.dlt[1], lane);
-            energy = (ep + ee) * vdown;
-            if (energy > 0.0 && isfinite(energy)) {
-                scale = (energy > budget) ? budget / energy : 1.0;
-            } else {
-                __syncwarp();
-                for (int j = lane; j < NB; j += 32) {
-                    sm.dlt[0][j] = 0.0;
-                    sm.dlt[1][j] = 0.0;
+        if (warp < 2) {
+            // X_cr = P_cr / P_th with E_cr above xcr_pmin (tracer_dsa_xcr_proton)
+            double e = 0.0;
+            for (int j = lane; j < NB; j += 32)
+                if (A.p[0][j] >= prm.xcr_pmin_pmc) e += ekin_erg(A.p[0][j], 0) * Np[j * A.js] * A.dp[0][j];
+            const double ecr = warp_sum(e) / vdown;
+            const double pth = rho1 * kKbCgs * k.temp / (prm.mu_mol * kMpG);
+            double xcr = 0.0;
+            if (pth > 0.0 && isfinite(ecr / 3.0) && isfinite(pth) && ecr / 3.0 > 0.0) xcr = (ecr / 3.0) / pth;
+            double eta_int = 0.0;
+            const int ii = prm.eta_model_initial, ir = prm.eta_model_reacc;
+            if (ii >= 0 && ii < 8 && ir >= 0 && ir < 8) {
+                const double ei = dsa_eta(mach, ii), er = dsa_eta(mach, ir);
+                const double x0 = c_models[ir].xcr0;
+                if (x0 <= 0.0) {
+                    eta_int = ei;
+                } else {
+                    const double wgt = fmin(fmax(xcr / x0, 0.0), 1.0);
+                    eta_int = (1.0 - wgt) * ei + wgt * er;
                 }
             }
+            double extra = eta_int - dsa_eta(mach, ii);
+            if (extra < 0.0 || !isfinite(extra)) extra = 0.0;
+            const double budget = extra * 0.5 * mass_g * u1 * u1;
+            if (budget > 0.0) {
+                const double es = reacc_positive(A, warp, warp ? Ne : Np, vdown, q, warp ? pmin_e : pmin_p, sm.dlt[warp], lane);
+                if (lane == 0) sm.e_dlt[warp] = es;
+            }
+            if (threadIdx.x == 0) sm.budget = budget;
         }
-        __syncwarp();
+        __syncthreads();
+        const double budget = sm.budget;
+        bool none = true;
+        if (budget > 0.0) {
+            energy = (sm.e_dlt[0] + sm.e_dlt[1]) * vdown;
+            if (energy > 0.0 && isfinite(energy)) {
+                scale = (energy > budget) ? budget / energy : 1.0;
+                none = false;
+            }
+        }
+        if (none) {   // each thread the bins that it applies below
+            for (int j = threadIdx.x; j < NB; j += kDsaThreads) {
+                sm.dlt[0][j] = 0.0;
+                sm.dlt[1][j] = 0.0;
+            }
+        }
     } else if (A.reacc == 2) {
-        reacc_convolution(A, 0, Np, vup, vdown, q, pmin_p, sm.dlt[0], lane);
-        reacc_convolution(A, 1, Ne, vup, vdown, q, pmin_e, sm.dlt[1], lane);
-        __syncwarp();
-        const double cp = delta_edens(A, 0, sm.dlt[0], pmin_p, lane);
-        const double ce = delta_edens(A, 1, sm.dlt[1], pmin_e, lane);
+        const bool capped = prm.reacc_eta_cap > 0.0 && isfinite(prm.reacc_eta_cap);
+        if (warp < 2) {
+            const double *N = warp ? Ne : Np;
+            const double pmin = warp ? pmin_e : pmin_p;
+            reacc_convolution(A, warp, N, vup, vdown, q, pmin, sm.dlt[warp], lane);
+            __syncwarp();
+            const double cs = delta_edens(A, warp, sm.dlt[warp], pmin, lane);
+            double as = 0.0;
+            if (capped) as = reacc_adiabatic(A, warp, N, vup, vdown, k.ratio, pmin, sm.ad[warp], lane);
+            if (lane == 0) {
+                sm.e_dlt[warp] = cs;
+                sm.e_ad[warp] = as;
+            }
+        }
+        __syncthreads();
+        const double cp = sm.e_dlt[0], ce = sm.e_dlt[1];
         energy = (cp + ce) * vdown;
         scale = 1.0;
-        if (prm.reacc_eta_cap > 0.0 && isfinite(prm.reacc_eta_cap)) {
+        if (capped) {
             const double budget = prm.reacc_eta_cap * 0.5 * mass_g * u1 * u1;
-            const double ap = reacc_adiabatic(A, 0, Np, vup, vdown, ratio, pmin_p, sm.ad[0], lane);
-            const double ae = reacc_adiabatic(A, 1, Ne, vup, vdown, ratio, pmin_e, sm.ad[1], lane);
+            const double ap = sm.e_ad[0], ae = sm.e_ad[1];
             const double nonad = (cp + ce - ap - ae) * vdown;
             if (nonad > 0.0 && isfinite(nonad) && budget > 0.0 && isfinite(budget)) {
                 if (nonad > budget) scale = budget / nonad;
-                for (int j = lane; j < NB; j += 32) {
+                for (int j = threadIdx.x; j < NB; j += kDsaThreads) {   // each thread the bins that it applies below
                     sm.dlt[0][j] = sm.ad[0][j] + scale * (sm.dlt[0][j] - sm.ad[0][j]);
                     sm.dlt[1][j] = sm.ad[1][j] + scale * (sm.dlt[1][j] - sm.ad[1][j]);
                 }
                 energy = (ap + ae + scale * (cp + ce - ap - ae)) * vdown;
             }
         }
-        __syncwarp();
-        if (A.dis && lane == 0) A.dis[t] = 1;
+        if (A.dis && threadIdx.x == 0) A.dis[t] = 1;
     }
 
     // apply: fresh sources, then the reacceleration deltas (from the
@@ -468,7 +510,7 @@ __global__ void __launch_bounds__(kDsaWarps * 32) dsa_inject_kernel(DsaArgs A)
     const double inv_dt = state ? 1.0 : 1.0 / A.dt_gyr;
     const double s_re = (A.reacc == 2) ? 1.0 : scale;
     const double *gp = A.dsa_p, *ge = A.dsa_p + NB;
-    for (int j = lane; j < NB; j += 32) {
+    for (int j = threadIdx.x; j < NB; j += kDsaThreads) {
         double vp = Op[j * A.js], ve = Oe[j * A.js];
         if (inj_p && fresh_p) {
             const double src = source_dp(A_p, pmin_p, q, prm.pmax_p_mc, gp[j]);
@@ -487,7 +529,23 @@ __global__ void __launch_bounds__(kDsaWarps * 32) dsa_inject_kernel(DsaArgs A)
     }
     bool applied = (inj_p && fresh_p) || (inj_e && fresh_p && fresh_e);
     if (reacc && scale > 0.0 && isfinite(energy) && fabs(energy) > 0.0) applied = true;
-    if (applied && lane == 0) atomicAdd(A.count, 1u);
+    if (applied && threadIdx.x == 0) atomicAdd(A.count, 1u);
+}
+
+__global__ void __launch_bounds__(kDsaThreads, 3) dsa_inject_kernel(const __grid_constant__ DsaArgs A)
+{
+    __shared__ DsaSmem sm;
+    __shared__ unsigned shocked;
+    const int t0 = blockIdx.x * A.per_block;
+    if (threadIdx.x < 32) {
+        const int t = t0 + threadIdx.x;
+        DsaShock k;
+        const bool hit = threadIdx.x < A.per_block && t < A.ntracer && dsa_shock(A, t, k);
+        const unsigned m = __ballot_sync(kFull, hit);
+        if (threadIdx.x == 0) shocked = m;
+    }
+    __syncthreads();
+    for (unsigned m = shocked; m; m &= m - 1) dsa_tracer(A, t0 + __ffs(m) - 1, sm);
 }
 
 }  // namespace
@@ -537,6 +595,7 @@ int dsa_inject(Context &c, const CromaB200Shocks *sh, double density_unit, doubl
     A.dsa_mach = dev[7]; A.dsa_pre_density = dev[8]; A.dsa_flux = dev[9];
     A.has_dsa = sh->has_dsa;
     A.ntracer = n;
+    A.per_block = n / kDsaSpread < 1 ? 1 : (n / kDsaSpread > kDsaTracers ? kDsaTracers : n / kDsaSpread);
     A.density_unit = density_unit;
     A.dt_gyr = dt_gyr;
     A.mode = mode;
@@ -562,12 +621,7 @@ int dsa_inject(Context &c, const CromaB200Shocks *sh, double density_unit, doubl
     }
     CROMA_CUDA(cudaMemsetAsync(c.d_dis, 0, (size_t)n, c.stream));
     CROMA_CUDA(cudaMemsetAsync(c.d_dsa_count, 0, sizeof(unsigned), c.stream));
-    constexpr size_t smem = kDsaWarps * sizeof(DsaSmem);
-    // set once per process; thread-safe (function-local static initialisation)
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(dsa_inject_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    CROMA_CUDA(attr);
-    dsa_inject_kernel<<<(n + kDsaWarps - 1) / kDsaWarps, kDsaWarps * 32, smem, c.stream>>>(A);
+    dsa_inject_kernel<<<(n + A.per_block - 1) / A.per_block, kDsaThreads, 0, c.stream>>>(A);
     CROMA_CUDA(cudaGetLastError());
     c.last_launches += 1;
     unsigned cnt = 0;
