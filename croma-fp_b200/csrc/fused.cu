@@ -2240,54 +2240,164 @@ cudaError_t launch_order(cudaStream_t st, int nt, const int *nsub, unsigned *bin
     return cudaGetLastError();
 }
 
-// Per-step kernel (the plain path): warp w of block b advances tracer
-// t0 + b * kWarps + w through the sub-steps of segment slot g0 with the
-// reference's per-step data contract -- every sub-step reads the rows a, b, c
-// of its on/off set, the source and N from memory, solves M N' = N + dt src
-// with the pivots recomputed (tracer_fp_cpu_evolve, src/tracer_fp_cpu.c:149-190;
-// fp_thomas_solve_ws, src/fp_shared_core.c:226-257) and writes N back.
-template <int S, bool SRC>
-__global__ void __launch_bounds__(kWarps * 32, (NB <= 256 ? 20 : 12)) plain_steps_kernel(FusedParams P)
+// Per-step kernel (the plain path): a block of one warp advances a tracer
+// through the sub-steps of segment slot g0 with the reference's per-step data
+// contract -- every sub-step reads the rows a, b, c of its on/off set from
+// memory, solves M N' = N + dt src with the pivots recomputed
+// (tracer_fp_cpu_evolve, src/tracer_fp_cpu.c:149-190; fp_thomas_solve_ws,
+// src/fp_shared_core.c:226-257) and writes N back.
+// The rows come through shared memory, copied across the lanes in 16-byte
+// pieces while the sub-step before is solved; lane l's pieces sit where the
+// lanes' reads of their own rows meet no bank twice.  The scans' shuffles (some
+// 40 of 64 bits a sub-step) and their latency bound it.  Before (each lane
+// loading its rows, half a cache line apart, as the sub-step began; the source
+// and all scan multipliers in registers) and now, both species, 512 bins 58.1 ->
+// 40.0 ms a snapshot of 16,384 tracers and 3.06 -> 2.78 ms of 64, 256 bins 19.8
+// -> 18.3 and 2.28 -> 2.07, 128 bins 11.3 -> 11.1 and 1.91 -> 1.70.  Sixteen
+// rows a lane and two or four systems a warp, with half the shuffles, took 22.0
+// and 11.5 ms at 256 and 128 bins: too few warps for the longer chains.
+constexpr int kPlainBlocks = NB <= 128 ? 24 : (NB <= 256 ? 20 : 12);   // per SM
+__device__ __forceinline__ int plain_piece(int c) { return c ^ ((c >> 3) & (kR / 2 - 1)); }
+__device__ __forceinline__ void plain_read(const double *buf, int lane, double v[kR])
 {
-    const int w = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int tl = blockIdx.x * kWarps + w;
-    if (tl >= P.nt) return;
-    const int t = P.t0 + tl;
-    const SnapArgs &a = P.a;
+#pragma unroll
+    for (int j = 0; j < kR / 2; j++) {
+        const double2 x = *reinterpret_cast<const double2 *>(buf + 2 * plain_piece(lane * (kR / 2) + j));
+        v[2 * j] = x.x;
+        v[2 * j + 1] = x.y;
+    }
+}
+template <int S, bool SRC>
+__global__ void __launch_bounds__(32, kPlainBlocks) plain_steps_kernel(const __grid_constant__ FusedParams P)
+{
+    constexpr int R = kR, H2 = R / 2;
+    __shared__ __align__(16) double buf[(SRC ? 4 : 3) * NB];   // a, b, c, the source
+    const int lane = threadIdx.x, tl = blockIdx.x, t = P.t0 + tl;
     const SegPre *__restrict__ pre = P.pre + tl;
     const int flags = pre->flags;
     if (!(flags & kPreActive)) return;
-    const int windowed = (flags & kPreWindowed) ? 1 : 0;
-    const int sl = pre->sl, el = pre->el, steps = pre->steps;
+    const bool windowed = flags & kPreWindowed;
+    const int steps = pre->steps, sl = windowed ? pre->sl : 0, el = windowed ? pre->el : steps;
     const double dt = pre->dt;
-    const int row0 = lane * kR;
-    double *Nrow = (S == 0 ? a.crp : a.cre) + (size_t)t * NB + row0;
-    const double *src = nullptr;
-    if (SRC) src = (S == 1 && P.inje) ? P.inje + (size_t)tl * NB : ((S == 0) ? a.qpi : a.qepri) + (size_t)t * NB;
-    Coef<SRC> F;
-    double N[kR];
+    double *Nrow = (S == 0 ? P.a.crp : P.a.cre) + (size_t)t * NB + lane * R;
+    auto fetch = [&](int istep) {   // the rows of a sub-step's set
+        const int set = istep >= sl && istep < el ? 0 : 1;
+        if (set >= P.sets) return false;   // no off set in the workspace
+        const double *f = fac_ptr(P, S, 0, set, tl);
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) {
+            const int c = i * 32 + lane;
+#pragma unroll
+            for (int k = 0; k < 3; k++) cp_async16(buf + k * NB + 2 * plain_piece(c), f + k * NB + 2 * c, true);
+        }
+        return true;
+    };
+    if (SRC) {
+        const double *src = (S == 1 && P.inje) ? P.inje + (size_t)tl * NB : (S == 0 ? P.a.qpi : P.a.qepri) + (size_t)t * NB;
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) {
+            const int c = i * 32 + lane;
+            cp_async16(buf + 3 * NB + 2 * plain_piece(c), src + 2 * c, true);
+        }
+    }
+    bool there = steps > 0 && fetch(0);
+    double N[R];
+#pragma unroll
+    for (int r = 0; r < R; r += 4) ld4(Nrow + r, N + r);
 #pragma unroll 1
     for (int istep = 0; istep < steps; istep++) {
-        const int set = (!windowed || (istep >= sl && istep < el)) ? 0 : 1;
-        if (set >= P.sets) {   // no off set in the workspace: report, leave N as it is
-            if (lane == 0) atomicOr(a.err, kErrBadInput);
-            return;
+        if (!there) {   // report, leave N as it is
+            if (lane == 0) atomicOr(P.a.err, kErrBadInput);
+            break;
         }
-        // rows a, b, c of the set: A <- a, inv <- b, q <- c, then the pivots
-        load_rows(fac_ptr(P, S, 0, set, tl), lane, F.h, F.inv, F.q);
-#pragma unroll
-        for (int r = 0; r < kR; r += 4) ld4(Nrow + r, N + r);
-        const unsigned err = pivot_rows<kR, 32>(F.h, F.inv, F.q, lane);
+        double A[R], B[R], C[R];
+        cp_async_wait_all();
+        __syncwarp();
+        plain_read(buf, lane, A);
+        plain_read(buf + NB, lane, B);
+        plain_read(buf + 2 * NB, lane, C);
+        __syncwarp();   // the buffer is read
+        there = istep + 1 < steps && fetch(istep + 1);
+        const unsigned err = pivot_rows<R, 32>(A, B, C, lane);
         if (__any_sync(kFull, err != 0)) {
-            if (lane == 0) atomicOr(a.err, kErrSingular);
-            return;
+            if (lane == 0) atomicOr(P.a.err, kErrSingular);
+            break;
         }
-        finish_coef<SRC>(F, src, dt, lane);
-        substep<SRC>(F, N);
+        if (lane == 0) A[0] = 0.0;
+        if (lane == 31) C[R - 1] = 0.0;
+        // y = (N + dt src) / d
+        if (SRC) {
+            double v[R];
+            plain_read(buf + 3 * NB, lane, v);
 #pragma unroll
-        for (int r = 0; r < kR; r += 4) st4(Nrow + r, N + r);
+            for (int r = 0; r < R; r++) N[r] = fma(N[r], B[r], (dt * v[r]) * B[r]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) N[r] *= B[r];
+        }
+        // forward: z_i = y_i + h_i z_{i-1}, two half-length chains a lane
+        double alo = 0.0, ahi = 0.0, hlo = 1.0, hhi = 1.0;
+#pragma unroll
+        for (int r = 0; r < H2; r++) {
+            alo = fma(A[r], alo, N[r]);
+            ahi = fma(A[r + H2], ahi, N[r + H2]);
+            hlo *= A[r];
+            hhi *= A[r + H2];
+        }
+        double acc = fma(hhi, alo, ahi), m = hlo * hhi;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double u = sup(acc, off), mu = sup(m, off);
+            if (lane >= off) {
+                acc = fma(m, u, acc);
+                m *= mu;
+            }
+        }
+        double cin = sup(acc, 1);
+        cin = lane > 0 ? cin : 0.0;
+        double plo = cin, phi = fma(hlo, cin, alo);
+#pragma unroll
+        for (int r = 0; r < H2; r++) {
+            plo = fma(A[r], plo, N[r]);
+            phi = fma(A[r + H2], phi, N[r + H2]);
+            N[r] = plo;
+            N[r + H2] = phi;
+        }
+        // back substitution: x_i = z_i + q_i x_{i+1}
+        alo = ahi = 0.0;
+        double qlo = 1.0, qhi = 1.0;
+#pragma unroll
+        for (int r = H2 - 1; r >= 0; r--) {
+            alo = fma(C[r], alo, N[r]);
+            ahi = fma(C[r + H2], ahi, N[r + H2]);
+            qlo *= C[r];
+            qhi *= C[r + H2];
+        }
+        acc = fma(qlo, ahi, alo);
+        m = qlo * qhi;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double d = sdn(acc, off), md = sdn(m, off);
+            if (lane + off < 32) {
+                acc = fma(m, d, acc);
+                m *= md;
+            }
+        }
+        double cout = sdn(acc, 1);
+        cout = lane < 31 ? cout : 0.0;
+        phi = cout;
+        plo = fma(qhi, cout, ahi);
+#pragma unroll
+        for (int r = H2 - 1; r >= 0; r--) {
+            phi = fma(C[r + H2], phi, N[r + H2]);
+            plo = fma(C[r], plo, N[r]);
+            N[r + H2] = phi;
+            N[r] = plo;
+        }
+#pragma unroll
+        for (int r = 0; r < R; r += 4) st4(Nrow + r, N + r);
     }
+    cp_async_wait_all();   // rows asked for before a singular system's end
 }
 
 // The per-segment scalars of every (slot, tracer) of the chunk, one thread
@@ -2692,10 +2802,9 @@ int tune_steps(Context &ctx, const FusedParams &P, bool src)
 template <int S>
 cudaError_t launch_steps(Context &ctx, const FusedParams &P, bool src, bool perstep)
 {
-    const int blocks = (P.nt + kWarps - 1) / kWarps;
     if (perstep) {
-        if (src) plain_steps_kernel<S, true><<<blocks, kWarps * 32, 0, ctx.stream>>>(P);
-        else plain_steps_kernel<S, false><<<blocks, kWarps * 32, 0, ctx.stream>>>(P);
+        if (src) plain_steps_kernel<S, true><<<P.nt, 32, 0, ctx.stream>>>(P);
+        else plain_steps_kernel<S, false><<<P.nt, 32, 0, ctx.stream>>>(P);
         return cudaGetLastError();
     }
     if (ctx.cfg.path == CROMA_PATH_FUSED_FP32R) {
