@@ -236,9 +236,8 @@ int fused_reserve(Context &ctx, int cap);
 // on path CROMA_PATH_*
 double fused_workspace_bytes(const ModelParams &mp, int cap, double workspace_cap, int path);
 int run_fused(Context &ctx, const SnapArgs &a);
-// the autotuner's choice for a species: solver (0 scan, 1 FP32-refined scan,
-// 2 PCR, 3 scan with its constants in shared memory) and warps per block;
-// returns 1 once tuned
+// the steps kernel of a species, by the autotuner or by rule: its solver (the
+// kSolve* values) and tracers per block; returns 1 once chosen
 int tuning_info(const Context &ctx, int species, int *solver, int *wpb);
 // dsa.cu
 int set_dsa(Context &ctx, const CromaB200DsaParams *prm);
