@@ -61,8 +61,9 @@ constexpr int kPkTracers = 32 / kPkLanes;
 constexpr int kFacDoubles = 3 * NB;  // 1/d, a/d, c/d of one system
 // Per-segment scalars of one (segment slot, tracer): what the factor kernels
 // of both species need of the schedule's segment and of the background
-// interpolated to it, computed once by seg_pre_kernel.
-struct SegPre {
+// interpolated to it, computed once by seg_pre_kernel.  Kernels copy it to shared
+// memory 16 bytes at a time, which its members alone (8 bytes) do not align it for.
+struct alignas(16) SegPre {
     double n_gas, kbt, inv_kbt, log_n, adiab, synch_coeff, coulomb_coeff;
     double dt, dt_over_tloss_pref, dtT_e, alpha, dpp_inv;
     int flags;               // bit 0 active, 1 windowed, 2 interpolated, 3 "on" Dpp filled
@@ -520,7 +521,8 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
     double2 *tab = reinterpret_cast<double2 *>(smem_raw);
     __shared__ double g_warp[2][kFacWarps];        // least g of the filled and the off form, per warp's share
     __shared__ SegPre pre_next[2][kFacWarps * kPkTracers];   // scalars of the warp's systems, one unit ahead
-    static_assert(sizeof(SegPre) == 7 * 16 && G >= 7, "a group's lanes copy its SegPre 16 bytes each");
+    static_assert(sizeof(SegPre) == 7 * 16 && alignof(SegPre) >= 16 && G >= 7,
+                  "a group's lanes copy its SegPre 16 bytes each");
     __shared__ unsigned tmem_base;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (G - 1);
     if (w == 0) tmem_alloc<kFacColumns>(&tmem_base);
