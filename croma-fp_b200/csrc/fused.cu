@@ -38,6 +38,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "croma_bits.cuh"
 #include "croma_segment.cuh"
 
 namespace croma {
@@ -227,12 +228,6 @@ __device__ __forceinline__ void continuant_scan(double t00, double t01, double t
         th = 1.0;
         thp = 0.0;
     }
-}
-
-// |theta_i / theta_{i-1}| <= 1e-300, to its exponent
-__device__ __forceinline__ bool continuant_singular(double n, double th)
-{
-    return (__double2hiint(n) & 0x7fffffff) + (996 << 20) < (__double2hiint(th) & 0x7fffffff);
 }
 
 // Thomas pivots of the rows a, b, c of a system, in place: Bd <- 1/d, A <- a/d,
