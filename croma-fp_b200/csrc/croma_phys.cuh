@@ -210,7 +210,8 @@ CROMA_HD void face_weights(double w, double &wp, double &wm)
     }
 }
 
-// FP64 reciprocal for the factor and per-step kernels.  CUDA's IEEE division
+// FP64 reciprocal (and quot_nr, the quotient) of the factor and per-step kernels
+// and the IC integrals.  CUDA's IEEE division
 // is a called routine: on B200 one costs ~125-145 cycles of a warp's time and
 // two of them never overlap (measured: the same per-division time at 1, 4 or
 // 8 independent divisions per thread), so a chain of pivots or a row of
@@ -219,8 +220,10 @@ CROMA_HD void face_weights(double w, double &wp, double &wm)
 // e = 1 - x y, y <- y + y e (each step squares the relative error), which
 // reach the FP64 rounding level for normal x (tested against the exact
 // reciprocal in ulps).  Subnormal x is flushed (then 0 gives a NaN) and
-// 1/x below the normal range returns 0; the callers' operands are O(1)
-// denominators bounded away from both.  Host builds divide.
+// 1/x below the normal range returns 0; the callers' operands stay away from
+// both: face denominators between 0.09 and 1e3, seed photon energies (1e-30 to
+// 1e3) and their exponentials (to 1e90), and continuants, whose rescaling keeps
+// them below 2^1016.  Host builds divide.
 CROMA_HD double rcp_nr(double x)
 {
 #ifdef __CUDA_ARCH__
@@ -232,6 +235,24 @@ CROMA_HD double rcp_nr(double x)
     return fma(y, e, y);
 #else
     return 1.0 / x;
+#endif
+}
+
+// a / b in as many instructions as a * rcp_nr(b), which rounds twice: the
+// reciprocal is refined once, to some 2^-40, and the quotient formed with it
+// takes its own residual a - b v (Newton's iteration on the quotient), so that
+// what is left is the last addition's rounding, half an ulp (tested).  Operands
+// as for rcp_nr, the quotient and the residual normal.
+CROMA_HD double quot_nr(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    const double v = a * y;
+    return fma(fma(-b, v, a), y, v);
+#else
+    return a / b;
 #endif
 }
 

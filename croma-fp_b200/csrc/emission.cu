@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) ic_table_kernel(IcConsts k, int nbins, co
                 if (!(X > k.log10_90)) {
                     const double ex = exp(X) - 1.0;
                     n = ex < 1.0e-40 ? k.cmb_pref * e / (9.11e-28 * kC * kC * (1.0 + 0.5 * X + X / 6.0) / (1.38e-16 * Tcmb))
-                                     : k.cmb_pref * (e * e) * rcp_nr(ex);
+                                     : k.cmb_pref * quot_nr(e * e, ex);
                 }
                 f = C * ie * n;
             }

@@ -242,7 +242,11 @@ __device__ __forceinline__ void continuant_scan(double t00, double t01, double t
 // reciprocals theta_{i-1} / theta_i are independent of each other, where the
 // pivot recurrence itself waits for one reciprocal a row (66 cycles against 8).
 // A row's rounding errors are those of d = b - e / d, since only the ratio of
-// the last two continuants enters it.
+// the last two continuants enters it, as one rounded quotient: the product with a
+// rounded reciprocal doubled the spectra's error growth over 500 sub-steps (mean
+// 2-norm error against 80 bits, 21 runs of 64 tracers: 1.08 of the former
+// recurrence's, 1.00 with the quotient; no change in time but 1 % of the per-step
+// path's, 4466 -> 4515 us at 256 bins, 4,096 tracers).
 template <int R, int LANES>
 __device__ __forceinline__ unsigned pivot_rows(double A[R], double Bd[R], double Cc[R], int gl)
 {
@@ -272,7 +276,7 @@ __device__ __forceinline__ unsigned pivot_rows(double A[R], double Bd[R], double
     for (int r = 0; r < R; r++) {
         const double n = fma(Bd[r], th, -(A[r] * cprev * thp));
         if (continuant_singular(n, th)) err = kErrSingular;
-        const double inv = th * rcp_nr(n);
+        const double inv = quot_nr(th, n);
         cprev = Cc[r];
         Bd[r] = inv;
         A[r] *= inv;
@@ -422,7 +426,7 @@ __device__ __forceinline__ void face_weights_half(double w, double &wp, double &
     const double E = exp_tab_normal(aw < 1400.0 ? -0.5 * aw : -700.0);
     const double e2 = E * E, w2 = w * w;
     const double dser = fma(w2, fma(w2, 1.0 / 1920.0, 1.0 / 24.0), 1.0);
-    const double q = (series ? 1.0 : aw) * rcp_nr(series ? E * dser : 1.0 - e2);
+    const double q = quot_nr(series ? 1.0 : aw, series ? E * dser : 1.0 - e2);
     const double s = q * e2;
     wp = (w >= 0.0) ? q : s;
     wm = (w >= 0.0) ? s : q;
@@ -839,7 +843,7 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                 for (int i = 0; i < 4; i++) {
                     const double n = fma(vi[i], th, -(vh[i] * cp * thp));
                     bad |= continuant_singular(n, th);
-                    vi[i] = th * rcp_nr(n);
+                    vi[i] = quot_nr(th, n);
                     cp = vq[i];
                     vh[i] *= vi[i];
                     vq[i] *= vi[i];

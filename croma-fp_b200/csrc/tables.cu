@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kIcWarps * 32) ic_row_kernel(const double *p_e
             double e = 0.0, f = 0.0;
             if (k <= N) {
                 e = eps[k];
-                const double t = e * rcp_nr(gamma - e), kappa = t * i4;
+                const double t = quot_nr(e, gamma - e), kappa = t * i4;
                 if (!(kappa <= 0.0))
                     f = e * (2.0 * kappa * log(kappa) + (1.0 + 2.0 * kappa) * (1.0 - kappa) +
                              0.5 * t * e * ig * (1.0 - kappa));

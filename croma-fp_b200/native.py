@@ -88,6 +88,7 @@ def load_library(nb: int) -> C.CDLL:
     L.croma_b200_fp64_peak.argtypes = [P(_d)]
     L.croma_b200_rcp_check.argtypes = [C.c_longlong, _vp, _vp]
     L.croma_b200_exp_check.argtypes = [C.c_longlong, _vp, _vp]
+    L.croma_b200_quot_check.argtypes = [C.c_longlong, _vp, _vp, _vp]
     L.croma_b200_h5_shape.argtypes = [C.c_char_p, C.c_char_p, P(_i), P(C.c_longlong), _i, P(_i), P(_i)]
     L.croma_b200_h5_read_f64.argtypes = [C.c_char_p, C.c_char_p, C.c_longlong, C.c_longlong, _vp]
     L.croma_b200_h5_read_i64.argtypes = [C.c_char_p, C.c_char_p, C.c_longlong, C.c_longlong, _vp]
@@ -248,11 +249,13 @@ def background_prepare(raw: dict, params: dict, ctx=None, nb: int = 256, on_devi
     return None if on_device else out
 
 
-def _math_check(fn: str, x, nb: int):
+def _math_check(fn: str, nb: int, *operands):
     L = load_library(nb)
-    xa = _c(x)
-    out = np.empty_like(xa)
-    if getattr(L, fn)(xa.size, _p(xa), _p(out)) != 0:
+    xs = [_c(x) for x in operands]
+    out = np.empty_like(xs[0])
+    if any(x.shape != out.shape for x in xs):
+        raise ValueError("operands must have one shape")
+    if getattr(L, fn)(out.size, *(_p(x) for x in xs), _p(out)) != 0:
         raise CromaError(L.croma_b200_last_error().decode())
     return out
 
@@ -260,13 +263,19 @@ def _math_check(fn: str, x, nb: int):
 def rcp_check(x, nb: int = 256):
     """The device reciprocal of the factor and per-step kernels applied to
     the float64 array x (croma_b200_rcp_check)."""
-    return _math_check("croma_b200_rcp_check", x, nb)
+    return _math_check("croma_b200_rcp_check", nb, x)
 
 
 def exp_check(x, nb: int = 256):
     """The factor kernels' table-driven exponential applied to the float64
     array x (croma_b200_exp_check)."""
-    return _math_check("croma_b200_exp_check", x, nb)
+    return _math_check("croma_b200_exp_check", nb, x)
+
+
+def quot_check(x, y, nb: int = 256):
+    """The quotient x / y of the factor and per-step kernels applied to the
+    float64 arrays x and y (croma_b200_quot_check)."""
+    return _math_check("croma_b200_quot_check", nb, x, y)
 
 
 def _shocks_struct(shocks: dict):

@@ -416,6 +416,8 @@ int croma_b200_fp64_peak(double *tflops);
 int croma_b200_rcp_check(long long n, const double *x, double *out);
 /* The same for the factor kernels' table-driven exponential. */
 int croma_b200_exp_check(long long n, const double *x, double *out);
+/* The same for their quotient x / y (its own Newton form). */
+int croma_b200_quot_check(long long n, const double *x, const double *y, double *out);
 
 #ifdef __cplusplus
 }
