@@ -264,7 +264,7 @@ __device__ __forceinline__ unsigned pivot_rows(double A[R], double Bd[R], double
         t11 = t01;
         t00 = n00;
         t01 = n01;
-        if ((r & 7) == 7 || r == R - 1) {   // d < 2^127 cannot leave the range in eight rows
+        if ((r & 3) == 3) {   // d < 2^255 cannot leave the range in four rows
             const double sc = pow2_norm(t00, t01);
             t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
         }
@@ -283,7 +283,7 @@ __device__ __forceinline__ unsigned pivot_rows(double A[R], double Bd[R], double
         Cc[r] *= inv;
         thp = th;
         th = n;
-        if ((r & 7) == 7 && r < R - 1) {
+        if ((r & 3) == 3 && r < R - 1) {
             const double sc = pow2_norm(th, thp);
             th *= sc;
             thp *= sc;
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                         t11 = t01;
                         t00 = n00;
                         t01 = n01;
-                        if (r == 7) {   // d < 2^127 cannot leave the range in eight rows
+                        if (i == 3) {   // d < 2^255 cannot leave the range in four rows
                             const double sc = pow2_norm(t00, t01);
                             t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
                         }
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                     thp = th;
                     th = n;
                 }
-                if (kk == 1) {
+                if (kk < R / 4 - 1) {
                     const double sc = pow2_norm(th, thp);
                     th *= sc;
                     thp *= sc;
