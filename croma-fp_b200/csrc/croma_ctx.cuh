@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/croma_b200.h"
+#include "croma_once.cuh"
 #include "croma_phys.cuh"
 
 #ifndef CROMA_NB
@@ -198,6 +199,17 @@ void timed_end(Context &ctx, int kind, cudaEvent_t start);
 // other's queued work.  Freed blocks stay in the device's pool for the next
 // allocation.  Other streams use the memory only after an event recorded on
 // the context stream, and host copies go through the context stream too.
+// A kernel's dynamic shared memory above the default 48 KB, set on the current
+// device by the launch that needs it first there.
+template <class Kernel>
+inline cudaError_t allow_smem(OncePerDevice &once, Kernel *kernel, size_t bytes)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return once(dev, [=] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
+}
+
 cudaError_t dev_alloc_bytes(Context &c, void **p, size_t bytes);
 template <class T>
 inline cudaError_t dev_alloc(Context &c, T **p, size_t bytes)

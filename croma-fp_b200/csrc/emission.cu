@@ -650,8 +650,8 @@ template <int MT>
 cudaError_t launch_gemm_tile(const EmisGemm &G, cudaStream_t st)
 {
     constexpr size_t smem = sizeof(EmisGemmSmem<MT>);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(emission_gemm_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, emission_gemm_kernel<MT>, smem);
     if (attr != cudaSuccess) return attr;
     const long long blocks = ((long long)G.nrows + MT - 1) / MT * G.ntiles;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -882,9 +882,7 @@ int emission_run(Context &c, const double *bg, double z, double *eps_syn, double
         size_t bytes = e->sort_tmp_bytes;
         CROMA_CUDA(cub::DeviceRadixSort::SortPairs(e->d_sort_tmp, bytes, kb, vb, n, 0, 16, st));
         constexpr size_t smem = sizeof(SynRows);
-        static const cudaError_t attr =
-            cudaFuncSetAttribute(synch_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        CROMA_CUDA(attr);
+        static_assert(smem <= 48 * 1024, "dynamic shared memory without an attribute");
         // frequencies split over blocks until the chip (2 blocks an SM) is filled
         // twice; each block's own cost, its spectra, is that of one frequency
         const long long blocks = ((long long)n + kSynWarps - 1) / kSynWarps;

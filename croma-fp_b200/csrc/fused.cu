@@ -2121,8 +2121,8 @@ template <int S, bool SRC>
 cudaError_t launch_packed(cudaStream_t st, const FusedParams &P)
 {
     constexpr size_t smem = (size_t)kPkWarps * (SRC ? 4 : 3) * 512 * sizeof(double);
-    static const cudaError_t attr = cudaFuncSetAttribute(steps_packed_kernel<S, SRC>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, steps_packed_kernel<S, SRC>, smem);
     if (attr != cudaSuccess) return attr;
     const int per = kPkWarps * kPkTracers;
     steps_packed_kernel<S, SRC><<<(P.nt + per - 1) / per, kPkThreads, smem, st>>>(P);
@@ -2607,9 +2607,8 @@ __global__ void __launch_bounds__(256, 2) secondary_kernel(FusedParams P)
 cudaError_t launch_secondary(Context &ctx, const FusedParams &P)
 {
     constexpr size_t smem = sizeof(GemmSmem);
-    // set once per process; thread-safe (function-local static initialisation)
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(secondary_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, secondary_kernel, smem);
     if (attr != cudaSuccess) return attr;
     const long long rows = (long long)(P.g1 - P.g0) * P.nt;
     if (rows > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -2624,8 +2623,8 @@ cudaError_t launch_factor(Context &ctx, const FusedParams &P)
 {
     constexpr size_t smem = (size_t)kFacTabs * NB * sizeof(double2) + (S == 0 ? kFacWarps * kCoulWarp : 0) * sizeof(double);
     static_assert(2 * (smem + 8192) <= 227 * 1024, "two blocks per SM");
-    static const cudaError_t attr = cudaFuncSetAttribute(factor_kernel<S, ROWS>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static OncePerDevice once;
+    const cudaError_t attr = allow_smem(once, factor_kernel<S, ROWS>, smem);
     if (attr != cudaSuccess) return attr;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
@@ -2654,8 +2653,8 @@ cudaError_t launch_steps_variant(cudaStream_t st, const FusedParams &P, int trac
                       : SOLVER == kSolveScanRhs    ? (size_t)WPB * kRhsSmemDoubles * sizeof(double)
                                                    : 0;
     if (smem > 48 * 1024) {
-        static const cudaError_t attr = cudaFuncSetAttribute(steps_kernel<S, SRC, SOLVER, WPB>,
-                                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        static OncePerDevice once;
+        const cudaError_t attr = allow_smem(once, steps_kernel<S, SRC, SOLVER, WPB>, smem);
         if (attr != cudaSuccess) return attr;
     }
     steps_kernel<S, SRC, SOLVER, WPB><<<blocks, WPB * 32, smem, st>>>(P);

@@ -462,13 +462,12 @@ int ic_rows(Context &ctx, double z, double *d_out)
     CROMA_CUDA(cudaMemcpyAsync(d_outer, outer, (N + 1) * sizeof(double), cudaMemcpyHostToDevice,
                                ctx.stream));
     CROMA_CUDA(cudaEventRecord(ctx.ic_stage_ev[k], ctx.stream));
-    static const cudaError_t attr = cudaFuncSetAttribute(ic_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)((kIcMaxOuter + 1) * kIcRowBytes));
-    CROMA_CUDA(attr);
+    static_assert((kIcMaxOuter + 1) * kIcRowBytes + kIcWarps * sizeof(double) <= 48 * 1024,
+                  "dynamic shared memory without an attribute");
     ic_abscissae_kernel<<<N + 1, 256, 0, ctx.stream>>>(ctx.icc, d_outer, N, width, z, ctx.d_ic_work);
     CROMA_CUDA(cudaGetLastError());
-    ic_row_kernel<<<NB + 2, kIcWarps * 32, (N + 1) * kIcRowBytes, ctx.stream>>>(ctx.gt.s[1].p, ctx.h_pm1[1], ctx.h_pp1[1], d_outer, N, width,
-                                                            ctx.d_ic_work, d_out);
+    ic_row_kernel<<<NB + 2, kIcWarps * 32, (N + 1) * kIcRowBytes, ctx.stream>>>(
+        ctx.gt.s[1].p, ctx.h_pm1[1], ctx.h_pp1[1], d_outer, N, width, ctx.d_ic_work, d_out);
     CROMA_CUDA(cudaGetLastError());
     return 0;
 }
