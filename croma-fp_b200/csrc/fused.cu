@@ -2710,11 +2710,12 @@ int tridiag_env()
     return 0;
 }
 
-// The autotuner of runs below the packed kernel's line (and of PCR): on the
-// first chunk a context evolves, each admissible variant of the family
-// tune_family names runs the chunk's tracers (at most kTuneTracers) for their
-// first 16 sub-steps on a copy of their spectra, timed with CUDA events; the
-// fastest is kept for the context's species.  Results are recorded in
+// The autotuner of runs below the packed kernel's line, and of PCR at any size:
+// on the first chunk a context evolves, each variant of the family tune_family
+// names runs the chunk's tracers (fewer than 64; under PCR, whose one variant is
+// timed to be reported, at most kTuneTracers) for their first 16 sub-steps on a
+// copy of their spectra, timed with CUDA events; the fastest is kept for the
+// context's species.  Results are recorded in
 // ctx.tune.  CROMA_B200_STEPS_VARIANT = 0..8 fixes the variant (scan x1, scan
 // x2, shared scan x1, shared scan x2, PCR, rhs-shared scan x1, rhs-shared scan
 // x2, short-chain scan x1, short-chain scan x2) without calibrating, for
@@ -2732,11 +2733,14 @@ int fixed_variant_env()
 // Which runs take the packed kernel: all of the FP64 on-chip path from
 // kPackedMin tracers on, unless the environment asks for PCR or names a
 // variant.  The line is on the run's tracers, not the chunk's, so that no
-// result depends on how a run is cut into chunks.  At the line the packed
-// kernel gains 14 % of the sub-steps' time (128 bins, 64 tracers: 152 -> 131
-// us) and spares the calibration's launches and waits; below it a launch is a
-// few blocks that wait on one warp's chain in either form, and the tuned
-// variants, which the environment can still name, stay.
+// result depends on how a run is cut into chunks; across it a tracer's spectra
+// agree to rounding (a run of 63 is another arithmetic than one of 64).  The line
+// is not where the kernels cross.  A snapshot of both species, alone, by the
+// tuned variants and by the packed kernel (us): 1 tracer 445 and 387 (128 bins),
+// 505 and 451 (256), 520 and 514 (512); 63 tracers 447 and 414, 507 and 481, 533
+// and 537; the first snapshot, calibration included, 1260 and 480, 1360 and 560,
+// 890 and 640.  Below it the tuner stays because its record is part of the
+// interface (croma_b200_get_tuning: the times of a family's variants).
 constexpr int kPackedMin = 64;
 bool packed_rule(const Context &ctx, const FusedParams &P)
 {

@@ -390,10 +390,9 @@ int cuda_get_current_device_id(char *out, int len)
 
 // CROMA_CUDA_TRIDIAG as the reference reads it (src/fp_cuda_solver.cu:41-72):
 // "pcr" selects PCR for power-of-two row counts up to 512 (-1 otherwise),
-// "thomas" selects Thomas.  Unset, this library's solvers are Thomas (the
-// stateless batch solve) and, in the pipeline, the steps-kernel autotuner's
-// choice, which has picked the warp-scan Thomas over warp PCR on every
-// configuration measured; the stateless query then reports Thomas.
+// "thomas" selects Thomas.  Unset, this library's solvers are Thomas: the
+// stateless batch solve, and the pipeline's packed scan or, below 64 tracers,
+// warp scans.
 int fp_cuda_tridiag_uses_pcr(int nrow)
 {
     const char *e = getenv("CROMA_CUDA_TRIDIAG");
@@ -699,7 +698,7 @@ int run_tracer_pipeline(const FpCudaPipelineInput *in, const FpCudaOutputSchedul
         times->solve_ms = elapsed(e1, e2);
         times->d2h_ms = elapsed(e2, e3);
         times->total_ms = elapsed(e0, e3);
-        // which sub-step solver the steps-kernel autotuner runs for each species
+        // which sub-step solver each species' steps kernel ran
         int solver = 0;
         if (tuning_info(c, 0, &solver, nullptr)) times->used_pcr_proton = solver == 2;
         if (tuning_info(c, 1, &solver, nullptr)) times->used_pcr_electron = solver == 2;

@@ -328,9 +328,10 @@ int croma_b200_step_host(CromaB200Context *ctx, const CromaB200Snapshot *snap, c
  * constants live -- registers, partly shared memory (fewer registers, more
  * warps per SM), or with each row's right-hand-side scaling in shared memory
  * too -- and in tracers (warps) per block, 1 or 2.  On the first workspace
- * chunk a context evolves, per species, each of them runs the chunk's first
- * tracers (up to 16,384) for 16 sub-steps on a copy of their spectra, timed
- * with CUDA events, and the fastest is kept for the context.  Reported here:
+ * chunk a context evolves, per species, each of them runs the chunk's tracers
+ * for 16 sub-steps on a copy of their spectra, timed with CUDA events, and the
+ * fastest is kept for the context.  A tracer's spectra in a run of fewer than 64
+ * agree with those in a larger run to rounding, not bit for bit.  Reported here:
  * tuned (0 before the first snapshot), solver (0 scan, 1 FP32-refined scan, 2
  * PCR, 3 scan with shared-memory constants, 4 scan with the right-hand-side
  * scaling in shared memory, 5 short-chain scan, 6 packed scan), tracers per
