@@ -180,21 +180,28 @@ __global__ void assign_bucket_kernel(int n, const int *seg_incl, const int *sort
 // tracers before its own; the members are placed in tracer order by one warp.
 // Three radix sorts and their dozen small kernels took 30 us of GPU time and
 // some 25 launches at 64 tracers, 33 us at 999; this takes 3.7 and 7.3 us and
-// one.  Above that the block's table outgrows its shared memory.
+// one.  The line: 4,096 tracers take one block 32 us (43 us with uneven counts),
+// 4,097 take the sorts 145 (138).  The block's table would fit for 8,192, where it
+// is still ahead of the sorts, 58 us (74) against 145 (143), a snapshot alone 641 us
+// against 770, but the snapshot's own kernels cover less of it: uneven snapshots
+// in a row, of which the build is the longest chain, 362 us against 351.  Above that
+// the table outgrows a block's shared memory.
 constexpr int kBucketOneBlock = 4096;
 constexpr int kBucketThreads = 1024;
 
-__host__ __device__ __forceinline__ int bucket_table(int n)   // a power of two, at least 2 n
+__host__ __device__ constexpr int bucket_table(int n)   // a power of two, at least 2 n
 {
     int h = 64;
     while (h < 2 * n) h <<= 1;
     return h;
 }
 
-size_t bucket_smem(int n)   // keys and first tracers of the table, slots of the tracers
+constexpr size_t bucket_smem(int n)   // keys and first tracers of the table, slots of the tracers
 {
     return (size_t)bucket_table(n) * (sizeof(unsigned long long) + sizeof(int)) + (size_t)n * sizeof(int);
 }
+
+static_assert(bucket_smem(kBucketOneBlock) + 256 <= 227 * 1024, "a block's shared memory");
 
 // exclusive prefix sum of v over the block, and its total
 __device__ __forceinline__ int block_prefix(int v, int *warp_sums, int &total)
