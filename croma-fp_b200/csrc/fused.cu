@@ -37,6 +37,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "croma_bits.cuh"
 #include "croma_segment.cuh"
@@ -389,7 +390,12 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 // arithmetic): 128 registers, 16 warps per SM.  The face loop is unrolled by four
 // rows only, so that it stays in the instruction cache.  Rows with a vanishing
 // diffusion coefficient (kappa g <= 1e-200) have their own forms
-// (Chang_Cooper.c:66-184); a system that could meet them takes rows_general.
+// (Chang_Cooper.c:66-184); a warp with a system that could meet them takes a copy
+// of the face loop that knows them: snapshots of 4,096 tracers on a grid from p =
+// 10^-3.2 (both species) 0.80 ms at 128 bins and 1.60 at 256, on the ordinary grid
+// 0.77 and 1.57; those systems' rows one by one, each row's terms formed three
+// times, 2.51 and 6.63, a warp per system before the packed layout 1.71 and 2.24.
+// The copy costs the other calls 0.3 to 0.7 %.
 //
 // Measured, before (a warp per system at every bin count, coefficients staged
 // in shared memory, a reciprocal a row in the serial chain of the pivots) and
@@ -426,88 +432,10 @@ __device__ __forceinline__ void face_weights_half(double w, double &wp, double &
     const double E = exp_tab_normal(aw < 1400.0 ? -0.5 * aw : -700.0);
     const double e2 = E * E, w2 = w * w;
     const double dser = fma(w2, fma(w2, 1.0 / 1920.0, 1.0 / 24.0), 1.0);
-    const double q = quot_nr(series ? 1.0 : aw, series ? E * dser : 1.0 - e2);
+    const double q = quot_nr(series ? 1.0 : aw, series ? E * dser : fma(-E, E, 1.0));
     const double s = q * e2;
     wp = (w >= 0.0) ? q : s;
     wm = (w >= 0.0) ? s : q;
-}
-
-// B = radp - 2 Dpp / p and C = Dpp at bin j, straight from the grid tables.
-template <int S>
-__device__ double2 terms_general(const FusedParams &P, const SegPre &p, double alpha, bool fill, double scale, int t, int j)
-{
-    const SpeciesTables &st = P.gt.s[S];
-    const double x = st.p[j];
-    double D = st.p2[j] * (1.0 / (4.0 * 1.0e+5));
-    if (fill) D = S == 0 ? st.p2[j] * p.dpp_inv * st.expE[j] * st.exp_cut[j] : st.p2[j] * p.dpp_inv * st.exp_cut[j];
-    D *= scale;
-    double radp;
-    if (S == 0) {
-        const double xp = P.gt.cp_Ep[j] * p.inv_kbt;
-        const double sum = coulomb_one(xp * (kMe / kMp)) + coulomb_one(xp) * (kMe / kMp);
-        const double thermal = 1.0 - p.kbt * P.gt.cp_inv2mpkin[j];
-        radp = (thermal < 0.0 ? 0.0
-                              : kGyr * kC / (kMp * kGeV) * sum * p.n_gas * P.gt.cp_inv_betap2[j] * thermal * 3.5e-29) +
-               p.adiab * x;
-    } else {
-        const size_t at = P.ic_stride ? (size_t)j * P.ic_stride + t : (size_t)j;
-        radp = p.synch_coeff * st.p2[j] + lerp(P.a.ic_curr[at], P.a.ic_next[at], alpha) +
-               p.coulomb_coeff * (1.0 + (P.gt.ce_logp[j] - p.log_n) * (1.0 / 74.8)) * P.gt.ce_inv_beta2[j] + p.adiab * x;
-    }
-    return make_double2(radp - st.two_over_p[j] * D, D);
-}
-
-// The raw rows a, b, c of the lane's 16 rows to out, with the forms of rows
-// and faces whose diffusion coefficient vanishes (cc_build_{left,interior,
-// right}, Chang_Cooper.c:66-184).  Rolled and slow: for systems that can meet
-// them only.
-template <int S>
-__device__ __noinline__ unsigned rows_general(const FusedParams &P, const SegPre &p, double alpha, bool fill, double scale,
-                                              int t, int gl, double *out)
-{
-    const SpeciesTables &st = P.gt.s[S];
-    unsigned err = 0;
-    auto face = [&](double2 l, double2 r, int j, double &wp, double &wm) {   // face j, between bins j and j + 1
-        wp = wm = 0.0;
-        if (fabs(l.y) > 1.0e-200) face_weights_fast((l.x + r.x) / (l.y + r.y) * st.dxf[j], wp, wm);
-    };
-#pragma unroll 1
-    for (int r = 0; r < kPkRows; r++) {
-        const int m = gl * kPkRows + r;
-        const double2 c0 = terms_general<S>(P, p, alpha, fill, scale, t, m);
-        const double2 cm = m > 0 ? terms_general<S>(P, p, alpha, fill, scale, t, m - 1) : make_double2(0.0, 0.0);
-        const double2 cp = m < NB - 1 ? terms_general<S>(P, p, alpha, fill, scale, t, m + 1) : make_double2(0.0, 0.0);
-        double wpm = 0.0, wmm = 0.0, wpc = 0.0, wmc = 0.0;
-        if (m > 0) face(cm, c0, m - 1, wpm, wmm);
-        if (m < NB - 1) face(c0, cp, m, wpc, wmc);
-        const double k = p.dt * st.inv_dx[m], D = S == 0 ? P.gt.sig_eff[m] * p.dt_over_tloss_pref : p.dtT_e;
-        const bool live = fabs(c0.y) > 1.0e-200;
-        double av = 0.0, bv, cv = 0.0;
-        const double fl = m > 0 ? 0.5 * (c0.y + cm.y) * st.inv_dxl[m] : 0.0;
-        const double fr = m < NB - 1 ? 0.5 * (c0.y + cp.y) * st.inv_dxr[m] : 0.0;
-        if (live) {
-            av = k * fl * wmm;
-            bv = 1.0 + k * (fl * wpm + fr * wmc) + D;
-            cv = k * fr * wpc;
-            if (m == NB - 1 && isnan(av)) err |= kErrCcNan;
-        } else if (m == 0) {
-            bv = 1.0 + k * 0.0 + D;
-            cv = k * 1.0 * 0.5 * (c0.x + cp.x);
-        } else if (m == NB - 1) {
-            double dlt = 0.0;
-            if (fabs(cm.y) > 1.0e-200) dlt = face_delta((cm.x + c0.x) / (cm.y + c0.y) * (st.p[m] - st.p[m - 1]));
-            av = -dlt * 0.5 * (c0.x + cm.x) * k;
-            bv = 1.0 + k * (0.5 * (cm.x + c0.x)) + D;
-        } else {
-            // every delta the reference reads here is zero (Chang_Cooper.c:91-103)
-            bv = 1.0 + k * (0.5 * (c0.x + cm.x)) + D;
-            cv = k * 1.0 * 0.5 * (c0.x + cp.x);
-        }
-        __stcg(out + m, av);
-        __stcg(out + NB + m, bv);
-        __stcg(out + 2 * NB + m, cv);
-    }
-    return err;
 }
 
 // ROWS: stores the raw rows a, b, c for the per-step path, which factors them
@@ -679,20 +607,29 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
         };
         // Rows from the faces above them (cc_build_*, Chang_Cooper.c:66-184), into
         // TMEM, and the matrix of the continuants' recurrence over rows 1 .. 15.
-        // A lane's first row waits for its neighbour's last face.
+        // A lane's first row waits for its neighbour's last face.  FLOOR: with the
+        // forms of rows whose diffusion coefficient vanishes (Chang_Cooper.c:66-184:
+        // no flux through the face above, upwind differences of B in the row); a
+        // system whose rows are all above the floor gets the same bits from both,
+        // the roundings being written out.
         double t00 = 1.0, t01 = 0.0, t10 = 0.0, t11 = 1.0;
-        double a0, b0, c0, e1 = 0.0;
-        {
+        double a0, b0, e1;
+        auto face_rows = [&](auto floor) {
+            constexpr bool FLOOR = decltype(floor)::value;
             double2 gr = form[FT_GR * NB];
             double Bc = B_of(0, gr.x), Pl = 0.0, Ml = 0.0, cl = 0.0;   // flux times weights of the face below; c of the row below
             const double B_up = __shfl_down_sync(kFull, Bc, 1, G);
+            double Bl = 0.0;               // B of the row below
+            bool live0 = true;
+            auto dpp_of = [&](int r, double g2p) { return 0.5 * (kappa * g2p) * row[FT_X2P * NB + r * G].y; };
+            if (FLOOR) Bl = __shfl_up_sync(kFull, B_of(R - 1, form[FT_GR * NB + (R - 1) * G].x), 1, G);
 #pragma unroll 1
             for (int kk = 0; kk < R / 4; kk++) {
                 unsigned ua[8], ub[8], uc[8];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int r = 4 * kk + i;
-                    const double rf = gr.y;
+                    const double rf = gr.y, g2p = gr.x;
                     double Bn = B_up;
                     if (r < R - 1) {
                         gr = form[FT_GR * NB + (r + 1) * G];
@@ -701,17 +638,36 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                     const double2 fk = form[FT_FK * NB + r * G];
                     double wp, wm;
                     face_weights_half((Bc + Bn) * (rf * inv_kappa), wp, wm);
+                    bool live = true;
+                    double Dpp = 0.0;
+                    if (FLOOR) {
+                        Dpp = dpp_of(r, g2p);
+                        live = !general || fabs(Dpp) > 1.0e-200;
+                        wp = live ? wp : 0.0;
+                        wm = live ? wm : 0.0;
+                    }
                     const double F = kappa * fk.x;
                     const double Pu = F * wp, Mu = F * wm;
                     const double k = dt * fk.y;
-                    const double D = S == 0 ? row[FT_X2P * NB + r * G].x * s2 : pre.dtT_e;
-                    const double ar = k * Ml, br = 1.0 + k * (Pl + Mu) + D, cr = k * Pu;
+                    double ar = k * Ml, br = fma(k, __dadd_rn(Pl, Mu), 1.0), cr = k * Pu;
+                    if (FLOOR && !live) {
+                        const bool first = gl == 0 && r == 0, last = gl == G - 1 && r == R - 1;
+                        const double Bs = 0.5 * (Bc + Bl);
+                        ar = 0.0;
+                        br = first ? 1.0 : fma(k, Bs, 1.0);
+                        cr = last ? 0.0 : k * (0.5 * (Bc + Bn));
+                        if (last) {
+                            const double Dl = dpp_of(R - 2, form[FT_GR * NB + (R - 2) * G].x);
+                            if (fabs(Dl) > 1.0e-200) ar = -face_delta((Bl + Bc) / (Dl + Dpp) * (st.p[NB - 1] - st.p[NB - 2])) * Bs * k;
+                        }
+                    }
+                    br = S == 0 ? fma(row[FT_X2P * NB + r * G].x, s2, br) : br + pre.dtT_e;
                     pk_set(ua, i, ar);
                     pk_set(ub, i, br);
                     pk_set(uc, i, cr);
                     if (r == 0) {
                         b0 = br;
-                        c0 = cr;
+                        live0 = live;
                     } else {
                         const double e = ar * cl;
                         const double n00 = fma(br, t00, -(e * t10)), n01 = fma(br, t01, -(e * t11));
@@ -723,8 +679,9 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                             const double sc = pow2_norm(t00, t01);
                             t00 *= sc; t01 *= sc; t10 *= sc; t11 *= sc;
                         }
-                        if (r == R - 1 && gl == G - 1 && on && !general && isnan(ar)) err |= kErrCcNan;
+                        if (r == R - 1 && gl == G - 1 && on && live && isnan(ar)) err |= kErrCcNan;
                     }
+                    if (FLOOR) Bl = Bc;
                     cl = cr;
                     Bc = Bn;
                     Pl = Pu;
@@ -737,54 +694,15 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
             Pl = __shfl_up_sync(kFull, Pl, 1, G);
             Ml = __shfl_up_sync(kFull, Ml, 1, G);
             const double k0 = dt * form[FT_FK * NB].y;
-            a0 = gl > 0 ? k0 * Ml : 0.0;
-            b0 = gl > 0 ? fma(k0, Pl, b0) : b0;
+            a0 = gl > 0 && live0 ? k0 * Ml : 0.0;
+            b0 = gl > 0 && live0 ? fma(k0, Pl, b0) : b0;
             tmem_wait_st();   // chunk 0 is there before two of its columns are written again
             tmem_st2(tm, a0);
             tmem_st2(tm + 8, b0);
             e1 = __shfl_up_sync(kFull, cl, 1, G);   // c of the row below the lane's first
-        }
-        if (__any_sync(kFull, general)) {
-            // those systems' rows by their own forms, through the output slot
-            if (general) err |= rows_general<S>(P, pre, alpha, fill, scale, t, gl, out);
-            __syncwarp();
-            tmem_wait_st();
-#pragma unroll 1
-            for (int r = 0; r < R; r++) {
-                double v[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const unsigned col = tm + (r >> 2) * 24 + 8 * k + 2 * (r & 3);
-                    unsigned q0, q1;
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(q0), "=r"(q1) : "r"(col));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(q0), "+r"(q1));
-                    v[k] = __hiloint2double((int)q1, (int)q0);
-                    if (general) v[k] = __ldcg(out + k * NB + gl * R + r);
-                    __syncwarp();
-                    tmem_st2(col, v[k]);
-                }
-                if (general) {
-                    if (r == 0) {
-                        a0 = v[0];
-                        b0 = v[1];
-                        c0 = v[2];
-                        t00 = t11 = 1.0;
-                        t01 = t10 = 0.0;
-                    } else {
-                        const double cp = __ldcg(out + 2 * NB + gl * R + r - 1), e = v[0] * cp;
-                        const double n00 = fma(v[1], t00, -(e * t10)), n01 = fma(v[1], t01, -(e * t11));
-                        const double sc = pow2_norm(n00, n01);
-                        t10 = t00 * sc;
-                        t11 = t01 * sc;
-                        t00 = n00 * sc;
-                        t01 = n01 * sc;
-                    }
-                    e1 = gl > 0 ? __ldcg(out + 2 * NB + gl * R - 1) : 0.0;
-                }
-                __syncwarp();
-            }
-        }
-        (void)c0;
+        };
+        if (__builtin_expect(__any_sync(kFull, general), 0)) face_rows(std::true_type{});
+        else face_rows(std::false_type{});
         const double c_in = gl > 0 ? e1 : 0.0;
         tmem_wait_st();
         if (ROWS) {
