@@ -88,6 +88,7 @@ struct FusedParams {
     // [nb][ntracer] (stride = ntracer)
     int ic_stride;
     const double *eta_scale; // [ntracer] Dpp eta-cap scale of slot g0, or null (no cap)
+    int pack;                // systems a warp of the factor kernel takes together, 1 .. kPkTracers
     double *fac;             // [2 species][g1 - g0][sets][nt][3][nb]
     SegPre *pre;             // [g1 - g0][nt]
     double *np_seg;          // [g1 - g0][nt][nb] proton spectra at segment starts, or null
@@ -498,13 +499,13 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
     }
     // rows a, b, c of chunk k (four rows) of the warp's lanes: 8 columns each
     const unsigned tm = tmem_base + ((unsigned)((w & 3) * 32) << 16) + (w >> 2) * 128;
-    // A unit: kPkTracers segments of one tracer and one set, or, with fewer
-    // segments than that, those of several tracers; unit numbers run over the
-    // tracers first, so that segments beyond a tracer's last fall evenly on the
-    // warps, and over the sets last: most windowed segments need one of the two,
-    // and a warp whose systems all need none of its set leaves at once (28 to
-    // 25 us a slot at 10,000 windowed tracers).
-    const int nslot = P.g1 - P.g0, segs = min(nslot, kPkTracers), tracers = kPkTracers / segs;
+    // A unit: P.pack segments of one tracer and one set, or, with fewer segments
+    // than that, those of several tracers; unit numbers run over the tracers
+    // first, so that segments beyond a tracer's last fall evenly on the warps, and
+    // over the sets last: most windowed segments need one of the two, and a warp
+    // whose systems all need none of its set leaves at once (28 to 25 us a slot at
+    // 10,000 windowed tracers).
+    const int nslot = P.g1 - P.g0, segs = min(nslot, P.pack), tracers = P.pack / segs;
     const int nq = (P.nt + tracers - 1) / tracers, nblk = (nslot + segs - 1) / segs;
     const int units = nblk * nq * P.sets, stride = gridDim.x * kFacWarps;
     const int sub = (lane / G) / segs, off = (lane / G) - sub * segs;   // the group's place in the unit
@@ -548,7 +549,8 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
             if (gl == 0) atomicOr(a.err, kErrBadInput);
             on = false;
         }
-        if (!__any_sync(kFull, on)) continue;
+        const unsigned firsts = __ballot_sync(kFull, on && gl == 0);   // first lanes of the systems in use
+        if (!firsts) continue;
         const bool fill = set == 0 && (flags & kPreFill);
         const double scale = (set == 0 && P.mp.dpp_model != kDppOff && P.eta_scale) ? P.eta_scale[t] : 1.0;
         const double kappa = fill ? pre.dpp_inv * scale : (1.0 / (4.0 * 1.0e+5)) * scale;
@@ -566,19 +568,38 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
             s1 = pre.kbt;
             s2 = pre.dt_over_tloss_pref;
             // the Coulomb kernels of the warp's systems
+#pragma unroll 1
+            for (unsigned m = firsts; m; m &= m - 1) {
+                const int l0 = __ffs(m) - 1;
+                const double ik = __shfl_sync(kFull, pre.inv_kbt, l0);
+                double *to = coul + l0 / G * kCoulSys;
 #pragma unroll 2
-            for (int it = 0; it < R; it++) {
-                const int i = it * 32 + lane, sys = i / NB, j = i % NB;
-                const double ik = __shfl_sync(kFull, pre.inv_kbt, sys * G);
-                const double xp = reinterpret_cast<const double *>(tab + FT_X34 * NB)[j] * ik;
-                const double sum = coulomb_one(xp * (kMe / kMp)) + coulomb_one(xp) * (kMe / kMp);
-                coul[sys * kCoulSys + (j % R) * kCoulPitch + j / R] = sum;
+                for (int j = lane; j < NB; j += 32) {
+                    const double xp = reinterpret_cast<const double *>(tab + FT_X34 * NB)[j] * ik;
+                    const double sum = coulomb_one(xp * (kMe / kMp)) + coulomb_one(xp) * (kMe / kMp);
+                    to[(j % R) * kCoulPitch + j / R] = sum;
+                }
             }
             __syncwarp();
         } else {
             s0 = pre.synch_coeff;
             s1 = pre.coulomb_coeff * (1.0 - pre.log_n * (1.0 / 74.8));
             s2 = pre.coulomb_coeff * (1.0 / 74.8);
+            if (P.ic_stride) {   // the tracers' own IC rows
+#pragma unroll 1
+                for (unsigned m = firsts; m; m &= m - 1) {
+                    const int l0 = __ffs(m) - 1, ts = __shfl_sync(kFull, t, l0);
+                    const double as = __shfl_sync(kFull, alpha, l0);
+                    double *to = coul + l0 / G * kCoulSys;
+#pragma unroll 4
+                    for (int j = lane; j < NB; j += 32) {
+                        const size_t at = (size_t)j * P.ic_stride + ts;
+                        const double c = a.ic_curr[at], n = a.ic_next[at];
+                        to[(j % R) * kCoulPitch + j / R] = lerp(c, n, as);
+                    }
+                }
+                __syncwarp();
+            }
         }
         const double2 *form = row + (fill ? 0 : 2 * NB);
         const double *cs = coul + (lane / G) * kCoulSys + gl;
@@ -595,8 +616,7 @@ __global__ void __launch_bounds__(kFacWarps * 32, kFacBlocks) factor_kernel(cons
                     const double2 x34 = row[FT_X34 * NB + r * G];
                     ric = fma(al, x34.y, x34.x);
                 } else {
-                    const size_t at = (size_t)(gl * R + r) * P.ic_stride + t;
-                    ric = lerp(a.ic_curr[at], a.ic_next[at], alpha);
+                    ric = cs[r * kCoulPitch];
                 }
                 B = fma(s0, x01.x, ric);
                 B = fma(s1, x01.y, B);
@@ -2537,22 +2557,30 @@ cudaError_t launch_secondary(Context &ctx, const FusedParams &P)
 }
 
 template <int S, bool ROWS>
-cudaError_t launch_factor(Context &ctx, const FusedParams &P)
+cudaError_t launch_factor(Context &ctx, FusedParams &P)
 {
-    constexpr size_t smem = (size_t)kFacTabs * NB * sizeof(double2) + (S == 0 ? kFacWarps * kCoulWarp : 0) * sizeof(double);
-    static_assert(2 * (smem + 8192) <= 227 * 1024, "two blocks per SM");
+    constexpr size_t tables = (size_t)kFacTabs * NB * sizeof(double2), rows = (size_t)kFacWarps * kCoulWarp * sizeof(double);
+    static_assert(2 * (tables + rows + 8192) <= 227 * 1024, "two blocks per SM");
+    const size_t smem = tables + (S == 0 || P.ic_stride ? rows : 0);
     static OncePerDevice once;
-    const cudaError_t attr = allow_smem(once, factor_kernel<S, ROWS>, smem);
+    const cudaError_t attr = allow_smem(once, factor_kernel<S, ROWS>, tables + rows);
     if (attr != cudaSuccess) return attr;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const long long systems = (long long)P.nt * (P.g1 - P.g0) * P.sets;
     if (systems > 0x7fff0000LL) return cudaErrorInvalidValue;
-    long long blocks = (systems + kFacWarps * kPkTracers - 1) / (kFacWarps * kPkTracers);
     // the occupancy query counts one block per SM for any kernel that allocates
     // TMEM; kFacBlocks of these fit by registers, columns and shared memory
     const long long full = (long long)nsm * kFacBlocks;
+    // A warp takes several systems together only where there are more than warps:
+    // a launch below that lasts as long as one unit, whose Coulomb terms and IC rows
+    // are formed system by system.  Bucket calls of 64 tracers, protons and electrons:
+    // 128 bins 15.0 and 17.6 us, now 10.2 and 10.4; 256 bins 15.1 and 18.7, 11.4 and
+    // 12.4 (512 bins: one system a warp either way).
+    const long long pack = (systems + full * kFacWarps - 1) / (full * kFacWarps);
+    P.pack = pack < 1 ? 1 : (pack > kPkTracers ? kPkTracers : (int)pack);
+    long long blocks = (systems + kFacWarps * P.pack - 1) / (kFacWarps * P.pack);
     if (blocks > full) blocks = full;
     if (blocks < 1) return cudaSuccess;
     factor_kernel<S, ROWS><<<(unsigned)blocks, kFacWarps * 32, smem, ctx.stream>>>(P);
