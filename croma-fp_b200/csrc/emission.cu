@@ -362,10 +362,11 @@ __global__ void fold_weights_kernel(int nbins, int wpitch, const double *kern, c
 // positive, the linear blend otherwise, clamped ends at t = 0 and 1.
 // Bound by the exponentials' instructions: they run as exp_tab_normal, four
 // rows of a lane at a time, where all of a warp's blends are in its range
-// (131,072 tracers, 64 frequencies, 512 bins: 10.4 ms with the general exp, a
-// row at a time behind its branches; now 7.7 ms).  A run whose tracers alone
-// do not fill the chip splits the frequencies over more blocks: 1,500 tracers
-// (188 blocks) 978 us, now 136 us.
+// (131,072 tracers, 64 frequencies: 10.4 ms at 512 bins and 3.08 at 128 with the
+// general exp, a row at a time behind its branches; now 6.3 and 2.64 ms), at four
+// blocks an SM: with two, 7.7 and 3.35 ms, since a block waits at a barrier for
+// each frequency's rows.  A run whose tracers alone do not fill the chip splits the
+// frequencies over more blocks: 1,500 tracers (188 blocks) 916 us, now 98 us.
 constexpr int kSynWarps = 8;
 
 __device__ __forceinline__ void synch_plane(double bval_in, double logb_min, double inv_dlogb, int nlogb, int &ib,
@@ -399,7 +400,7 @@ struct SynRows {
     double L[2][3][NB];   // log K of the block's planes at this frequency and the next
 };
 
-__global__ void __launch_bounds__(kSynWarps * 32, 2) synch_sorted_kernel(
+__global__ void __launch_bounds__(kSynWarps * 32, 4) synch_sorted_kernel(
     int ntracer, int nfreq, int nlogb, double logb_min, double inv_dlogb, SynchPrefactor sp, const double *K,
     const double *logK, const int *order, const double *bfield, const double *cre, const double *dp, double *out)
 {
@@ -883,8 +884,8 @@ int emission_run(Context &c, const double *bg, double z, double *eps_syn, double
         CROMA_CUDA(cub::DeviceRadixSort::SortPairs(e->d_sort_tmp, bytes, kb, vb, n, 0, 16, st));
         constexpr size_t smem = sizeof(SynRows);
         static_assert(smem <= 48 * 1024, "dynamic shared memory without an attribute");
-        // frequencies split over blocks until the chip (2 blocks an SM) is filled
-        // twice; each block's own cost, its spectra, is that of one frequency
+        // frequencies split over blocks until the chip (4 blocks an SM) is filled;
+        // each block's own cost, its spectra, is that of one frequency
         const long long blocks = ((long long)n + kSynWarps - 1) / kSynWarps;
         const long long want = 4LL * sm_count() / blocks;
         const unsigned split = (unsigned)(want < 1 ? 1 : (want > s.nfreq ? s.nfreq : want));
