@@ -45,10 +45,14 @@ constexpr double kPiD = 3.14159265358979323846;
 // 3 busy warps an SM at 512 bins) and now, 5 % shocked: 131,072 tracers 1.82 ms
 // and 0.58, 1,500 tracers 205 us and 80.  Smaller runs take fewer tracers a
 // block, down to one: eight of 1,500 make some blocks take four shocks in turn
-// (178 us); one of 131,072 costs mostly block launches.
+// (178 us); one of 131,072 costs mostly block launches (so do 3,000 without any
+// shock: 37 and 45 us).  The other side of it, most tracers shocked: with
+// reacceleration, during which two warps of a block work, 40,000 tracers take 2.50
+// and 3.37 ms at 128 bins, 4.90 and 6.17 at 512 with all of them shocked, 1.23 and
+// 1.12, 3.36 and 2.04 with 30 %.
 constexpr int kDsaThreads = 256;
 constexpr int kDsaTracers = 8;
-constexpr int kDsaSpread = 2368;   // blocks, 16 an SM, before a block takes more than one tracer
+constexpr int kDsaSpread = 16;     // blocks an SM before a block takes more than one tracer
 
 struct DsaModelCoef {
     int family, reacc;
@@ -247,14 +251,6 @@ __device__ bool resolve_input(const DsaArgs &A, int t, double &mach, double &tem
     return true;
 }
 
-// Reacceleration deltas and adiabatic deltas of both species, the partial sums
-// of the Simpson integral and the species' energy sums.
-struct DsaSmem {
-    double dlt[2][NB], ad[2][NB];
-    double part[kDsaThreads / 32];
-    double e_dlt[2], e_ad[2], budget;
-};
-
 // What the injection of one shocked tracer starts from; false: it has none.
 struct DsaShock {
     double mach, temp, rho1, u1, ratio, u2, q, pmin_p, pmin_e, chi_e, mass_g, vup, vdown;
@@ -385,13 +381,21 @@ __device__ double reacc_adiabatic(const DsaArgs &A, int s, const double *N, doub
     return delta_edens(A, s, ad, pmin, lane);
 }
 
-// All threads of the block on tracer t.
-__device__ void dsa_tracer(const DsaArgs &A, int t, DsaSmem &sm)
+// The shocks of the block's tracers, the reacceleration and adiabatic deltas of
+// both species, the partial sums of the Simpson integral and the species' energy
+// sums.
+struct DsaSmem {
+    DsaShock shock[kDsaTracers];
+    double dlt[2][NB], ad[2][NB];
+    double part[kDsaThreads / 32];
+    double e_dlt[2], e_ad[2], budget;
+};
+
+// All threads of the block on tracer t and its shock k.
+__device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &sm)
 {
     const CromaB200DsaParams &prm = A.prm;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    DsaShock k;
-    if (!dsa_shock(A, t, k)) return;   // the same in all threads; true, as the caller found
     const double mach = k.mach, rho1 = k.rho1, u1 = k.u1, q = k.q, pmin_p = k.pmin_p, pmin_e = k.pmin_e;
     const double chi_e = k.chi_e, mass_g = k.mass_g, vup = k.vup, vdown = k.vdown;
     const int inj_p = prm.inject_species != 2, inj_e = prm.inject_species != 1;
@@ -539,13 +543,15 @@ __global__ void __launch_bounds__(kDsaThreads, 3) dsa_inject_kernel(const __grid
     const int t0 = blockIdx.x * A.per_block;
     if (threadIdx.x < 32) {
         const int t = t0 + threadIdx.x;
-        DsaShock k;
-        const bool hit = threadIdx.x < A.per_block && t < A.ntracer && dsa_shock(A, t, k);
+        const bool hit = threadIdx.x < A.per_block && t < A.ntracer && dsa_shock(A, t, sm.shock[threadIdx.x & (kDsaTracers - 1)]);
         const unsigned m = __ballot_sync(kFull, hit);
         if (threadIdx.x == 0) shocked = m;
     }
     __syncthreads();
-    for (unsigned m = shocked; m; m &= m - 1) dsa_tracer(A, t0 + __ffs(m) - 1, sm);
+    for (unsigned m = shocked; m; m &= m - 1) {
+        const int i = __ffs(m) - 1;
+        dsa_tracer(A, t0 + i, sm.shock[i], sm);
+    }
 }
 
 }  // namespace
@@ -595,7 +601,10 @@ int dsa_inject(Context &c, const CromaB200Shocks *sh, double density_unit, doubl
     A.dsa_mach = dev[7]; A.dsa_pre_density = dev[8]; A.dsa_flux = dev[9];
     A.has_dsa = sh->has_dsa;
     A.ntracer = n;
-    A.per_block = n / kDsaSpread < 1 ? 1 : (n / kDsaSpread > kDsaTracers ? kDsaTracers : n / kDsaSpread);
+    int nsm = 0;
+    CROMA_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    const int share = n / (kDsaSpread * (nsm < 1 ? 1 : nsm));
+    A.per_block = share < 1 ? 1 : (share > kDsaTracers ? kDsaTracers : share);
     A.density_unit = density_unit;
     A.dt_gyr = dt_gyr;
     A.mode = mode;
