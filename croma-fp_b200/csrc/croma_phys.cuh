@@ -59,10 +59,8 @@ struct SpeciesTables {
     const double *two_over_p;   // 2/p used in B = radp - 2 Dpp / p (fp_shared_core.c:2401)
     const double *expE;         // exp(-E/E_max) (protons; FP_Coef.c:699)
     const double *inv_dx;       // 1 / dp
-    const double *inv_dxl;      // 1 / (p[j] - p[j-1])   (j >= 1)
     const double *inv_dxr;      // 1 / (p[j+1] - p[j])   (j <= nb-2)
     const double *dxf;          // p[j+1] - p[j]         (j <= nb-2), face widths
-    const double *face_rf;      // dxf[j] / (g[j] + g[j+1]), g = p^2 expE exp(-1/p) (j <= nb-2)
     double pm1, pp1;
     double pm1_p2, pp1_p2, pm1_exp_cut, pp1_exp_cut;
     double expE_m1, expE_p1;    // exp(-m_p sqrt(1+p^2)/E_max) at the ghost edges
@@ -284,8 +282,7 @@ constexpr double kExpLlo = 0x1.abc9e3b39803fp-61;   // ln2 / 32 - kExpLhi
 
 #ifdef __CUDACC__
 // 2^(j/32) exp(r), j the low five bits of N: exp(x) = 2^(N >> 5) times it
-template <class Entry>
-__device__ __forceinline__ double exp_tab_fraction(double x, int &N, Entry entry)
+__device__ __forceinline__ double exp_tab_fraction(double x, int &N)
 {
     const double t = fma(x, kExpInvL, 0x1.8p52);
     const double n = t - 0x1.8p52;
@@ -297,7 +294,7 @@ __device__ __forceinline__ double exp_tab_fraction(double x, int &N, Entry entry
     double v = fma(1.0 / 120.0, r, 1.0 / 24.0);
     v = fma(1.0 / 720.0, r2, v);
     const double p = fma(fma(v, r2, u), r2, r);
-    const double tj = entry(N & 31);   // 2^(j/32)
+    const double tj = __ldg(&kExp2J[N & 31]);
     return fma(tj, p, tj);
 }
 #endif
@@ -306,7 +303,7 @@ CROMA_HD double exp_tab(double x)
 #ifdef __CUDA_ARCH__
     x = x < -746.0 ? -746.0 : (x > 709.0 ? 709.0 : x);   // a NaN passes through
     int N;
-    const double f = exp_tab_fraction(x, N, [](int j) { return __ldg(&kExp2J[j]); });
+    const double f = exp_tab_fraction(x, N);
     const int m = N >> 5, m1 = m >> 1, m2 = m - m1;
     const double s1 = __hiloint2double((m1 + 1023) << 20, 0), s2 = __hiloint2double((m2 + 1023) << 20, 0);
     return f * s1 * s2;
@@ -322,38 +319,13 @@ __device__ __forceinline__ bool exp_tab_normal_range(double x)   // false for a 
 {
     return (__double2hiint(x) & 0x7fffffff) < 0x40862000;
 }
-template <class Entry>
-__device__ __forceinline__ double exp_tab_normal(double x, Entry entry)
-{
-    int N;
-    const double f = exp_tab_fraction(x, N, entry);
-    return __hiloint2double(__double2hiint(f) + ((N & ~31) << 15), __double2loint(f));
-}
 __device__ __forceinline__ double exp_tab_normal(double x)
 {
-    return exp_tab_normal(x, [](int j) { return __ldg(&kExp2J[j]); });
+    int N;
+    const double f = exp_tab_fraction(x, N);
+    return __hiloint2double(__double2hiint(f) + ((N & ~31) << 15), __double2loint(f));
 }
 #endif
-
-// The same weights with one exponential and one division per face and no
-// divergent branch (the evolve kernels' form): exp(-w/2) is taken as
-// 1/exp(w/2), the exponential is exp_tab, the two quotients by the
-// denominator share one reciprocal (rcp_nr) and the series constants are
-// multiplied in.  Agrees with
-// face_weights to a few ulp.
-CROMA_HD void face_weights_fast(double w, double &wp, double &wm)
-{
-    const double aw = fabs(w);
-    const bool series = aw < 0.1;
-    const double w2 = w * w;
-    const double dser = 1.0 + w2 * (1.0 / 24.0) + (w2 * w2) * (1.0 / 1920.0);
-    const double e = exp_tab(series ? 0.5 * w : -aw);
-    const double q = (series ? 1.0 : aw) * rcp_nr(series ? e * dser : 1.0 - e);
-    const double s = q * e;
-    // series: wm = 1 / (e dser), wp = e / dser; otherwise big = q, small = q e
-    wp = series ? s * e : ((w >= 0.0) ? q : s);
-    wm = series ? q : ((w >= 0.0) ? s : q);
-}
 
 CROMA_HD double face_delta(double w)
 {

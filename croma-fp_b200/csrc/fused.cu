@@ -51,9 +51,6 @@ constexpr int kR = NB / 32;          // rows per lane
 // R lane + r) and those at a stride then touch distinct bank pairs.
 constexpr int kPitch = 32 + 16 / kR;
 constexpr int kSw = kPitch * kR;     // swizzled row-array length
-// One warp per block in the steps kernels: a finished tracer's slot is
-// refilled at once instead of when the slowest warp of its block ends.
-constexpr int kWarps = 1;            // warps per block
 constexpr unsigned kFull = 0xffffffffu;
 // Packed layout (factor and packed steps kernels): 16 rows a lane at every bin
 // count, so 8, 16 or 32 lanes hold a system and a warp 4, 2 or 1 of them.
@@ -129,7 +126,7 @@ __device__ __forceinline__ double sdn(double v, int d) { return __shfl_down_sync
 // loads and stores).  The lanes of a warp own 128-byte row blocks, so a
 // 16-byte access per lane would touch 32 sectors and use half of each (a
 // scalar access a quarter); 32 bytes per lane use every sector fully.  The
-// asm is volatile so that the per-step path's re-reads stay in its loop.
+// asm is volatile, so that loads and stores keep their order.
 // ld4_cg / st4_cg: L2 only (rows and sources); ld4 / st4: the default caching.
 __device__ __forceinline__ void ld4_cg(const double *p, double *v)
 {
@@ -423,8 +420,9 @@ constexpr int kCoulPitch = kPkLanes + 1;
 constexpr int kCoulSys = kPkRows * kCoulPitch;
 constexpr int kCoulWarp = kPkTracers * kCoulSys;
 
-// Chang-Cooper weights of a face (face_weights_fast's arithmetic, with one
-// exponential exp(-|w| / 2) for both of its branches).
+// Chang-Cooper weights of a face (face_weights, croma_phys.cuh) with one
+// exponential exp(-|w| / 2) for both branches and one quotient; agrees with it to
+// a few ulp.
 __device__ __forceinline__ void face_weights_half(double w, double &wp, double &wm)
 {
     const double aw = fabs(w);
@@ -1725,7 +1723,7 @@ __device__ __forceinline__ void pk_read(const double *buf, int k, int gl, double
 // and the warp advances all its groups by the smallest remaining run.  When
 // any group starts a run, all load their constants again (the others' are
 // what they were).  A group without work holds the identity (1/d = 1, the
-// rest 0), which leaves its rows as they are, bit for bit.
+// rest 0), which leaves finite rows as they are.
 template <int S, bool SRC>
 __global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams P)
 {
@@ -1875,7 +1873,7 @@ __global__ void __launch_bounds__(kPkThreads, 3) steps_packed_kernel(FusedParams
                     pgi = gi + 1;
                     pset = (steps > el || el == sl) ? 1 : 0;
                 }
-                if (pgi < P.g1 - P.g0) pk_fetch<S, SRC>(P, buf, pgi, pset, tl, gl);
+                if (pgi < P.g1 - P.g0 && pset < P.sets) pk_fetch<S, SRC>(P, buf, pgi, pset, tl, gl);
                 else pgi = -1;
                 walk.pgi[me] = pgi;
                 walk.pset[me] = pset;
