@@ -56,12 +56,12 @@ METRIC = "tracer-snapshot updates/s at <=1e-6 rel err vs FP64, chosen vs plain; 
 UNIT = "tracer-snapshot updates/s"
 SHOCK_KEYS = ("mach", "prestemp", "presden", "shock_side_code")
 # DRAM bytes (read + write) per tracer of one launch of each kernel, from the
-# ncu captures of this workload's kernels at 16,384 tracers
-# (profiles/*_full_pipeline_e_p_512.txt: DRAM rate x duration / 16,384).  Every
-# tracer moves its own rows, so a launch's traffic is this figure times the
-# tracers it processes.  steps: mean of the proton and electron launches;
-# plain_steps: the electron launch of one segment slot.
-NCU_DRAM_BYTES_PER_TRACER = {"steps": (272.2e3 + 271.0e3) / 2, "plain_steps": 23.7e3}
+# ncu captures of this workload's kernels at 4,096 tracers.  Every tracer moves
+# its own rows, so a launch's traffic is this figure times the tracers it
+# processes.  Means of the proton and electron launches (plain_steps: of one
+# segment slot).
+STEPS_PROFILE, PLAIN_PROFILE = "profiles/steps_packed_kernel_512.txt", "profiles/plain_steps_kernel_512.txt"
+NCU_DRAM_BYTES_PER_TRACER = {"steps": (266.9e3 + 272.0e3) / 2, "plain_steps": (16.8e3 + 21.2e3) / 2}
 
 
 def load_package():
@@ -620,10 +620,9 @@ def roofline_fused(cfg, nt, res, steps, fp64_peak, peaks, peak_kind):
     ms_total = res["ms"]
     return {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
             "frac": achieved / fp64_peak, "traffic": traffic,
-            "traffic_source": "ncu DRAM bytes per tracer-launch (profiles/steps_kernel_*_full_pipeline_e_p_512.txt) "
-                              "x tracers per launch",
+            "traffic_source": f"ncu DRAM bytes per tracer-launch ({STEPS_PROFILE}) x tracers per launch",
             "peak_source": "measured live: croma_b200_fp64_peak (FMA chains on every SM)",
-            "kernel": "steps_kernel (proton and electron launches per workspace chunk)",
+            "kernel": "steps_packed_kernel (proton and electron launches per workspace chunk)",
             "launches": ev_n, "kernel_ms_total": ev_ms, "share_of_step": ev_ms / ms_total,
             "alg_flops_per_launch": per_launch,
             "alg_flops_rule": "per tracer-snapshot: nsub x 2 species x nb x 11 (reference Thomas step)",
@@ -652,8 +651,7 @@ def roofline_plain(cfg, nt, res, steps, peaks, peak_kind):
                if cfg.nb == 512 else None)
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "peak_source": peak_kind,
-            "traffic_source": "ncu DRAM bytes per tracer-launch (profiles/plain_steps_kernel_electrons_full_pipeline_"
-                              "e_p_512.txt) x tracers per launch",
+            "traffic_source": f"ncu DRAM bytes per tracer-launch ({PLAIN_PROFILE}) x tracers per launch",
             "frac_meaning": "contract bytes (the reference's per-step data contract) per second; each warp runs "
                             "its slot's sub-steps back to back, so the per-step re-reads hit L2 and DRAM itself "
                             "sees a few per cent of these bytes (traffic)",
