@@ -1,5 +1,6 @@
 // dsa.cu -- per-snapshot DSA (diffusive shock acceleration) injection into the
-// device-resident tracer spectra, one block at a time per shocked tracer.
+// device-resident tracer spectra, one block at a time per shocked tracer,
+// or two of its warps where many are shocked.
 //
 // For every tracer whose shock fields pass the reference's checks the block
 //   1. resolves the upstream state (Mach number, temperature, density,
@@ -46,12 +47,16 @@ constexpr double kPiD = 3.14159265358979323846;
 // and 0.58, 1,500 tracers 205 us and 80.  Smaller runs take fewer tracers a
 // block, down to one: eight of 1,500 make some blocks take four shocks in turn
 // (178 us); one of 131,072 costs mostly block launches (so do 3,000 without any
-// shock: 37 and 45 us).  The other side of it, most tracers shocked: with
-// reacceleration, during which two warps of a block work, 40,000 tracers take 2.50
-// and 3.37 ms at 128 bins, 4.90 and 6.17 at 512 with all of them shocked, 1.23 and
-// 1.12, 3.36 and 2.04 with 30 %.
+// shock: 37 and 45 us).
+// Reacceleration keeps two warps busy, a species each.  So a block with three
+// shocked tracers and more (four without it, where only the waits at barriers are
+// saved) gives each to two of its warps, four at a time: 40,000 tracers, all
+// shocked, a warp per tracer, a block a tracer and now 2.51, 3.37 and 2.67 ms at 128
+// bins, 4.91, 6.17 and 4.04 at 512, without reacceleration 2.21, 2.57 and 2.25, 3.42,
+// 2.95 and 2.62; 5 % shocked the same as a block a tracer.
 constexpr int kDsaThreads = 256;
 constexpr int kDsaTracers = 8;
+constexpr int kDsaPairs = 4, kDsaPairsReacc = 3;   // shocked tracers of a block from which two warps take one each
 constexpr int kDsaSpread = 16;     // blocks an SM before a block takes more than one tracer
 
 struct DsaModelCoef {
@@ -178,25 +183,47 @@ __device__ __forceinline__ double warp_scan(double v, int lane)
     return v;
 }
 
+// The warps that work on one tracer: the whole block, or two of its warps.
+template <int WARPS>
+struct DsaTeam {
+    static constexpr int kThreads = WARPS * 32, kPerBlock = kDsaThreads / kThreads;
+    int tid, warp, index;   // thread and warp in the team, team in the block
+    __device__ DsaTeam() : tid(threadIdx.x % kThreads), warp(threadIdx.x % kThreads / 32), index(threadIdx.x / kThreads) {}
+    __device__ void sync() const
+    {
+        if (WARPS * 32 == kDsaThreads) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + index), "n"(WARPS * 32) : "memory");
+    }
+};
+
 // 4 pi m_p c^2 x Simpson integral of the energy integrand over [p_inj, p_max],
-// by the whole block (the arguments are the same in all of its threads)
-__device__ double proton_edens_unit(double pinj, double q, double pmax, double *part)
+// by a team (the arguments are the same in all of its threads): eight partial sums
+// of 32 lanes each, whatever the team, so that the result does not depend on it.
+template <int WARPS>
+__device__ double proton_edens_unit(double pinj, double q, double pmax, double *part, const DsaTeam<WARPS> &team)
 {
     if (pinj <= 0.0 || pmax <= 0.0 || pmax <= pinj) return 0.0;
     constexpr int nstep = 4000;
     const double h = (pmax - pinj) / (double)nstep;
-    double s = 0.0;
-    for (int i = 1 + threadIdx.x; i < nstep; i += kDsaThreads) {
-        const double p = pinj + h * (double)i;
-        s += ((i % 2) ? 4.0 : 2.0) * energy_integrand(p, pinj, q, pmax);
-    }
-    s = warp_sum(s);
-    __syncthreads();   // part's readers of the tracer before are done
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    s = 0.0;
+    double sums[8 / WARPS];
 #pragma unroll
-    for (int w = 0; w < kDsaThreads / 32; w++) s += part[w];
+    for (int k = 0; k < 8 / WARPS; k++) {
+        double s = 0.0;
+        for (int i = 1 + k * WARPS * 32 + team.tid; i < nstep; i += 256) {
+            const double p = pinj + h * (double)i;
+            s += ((i % 2) ? 4.0 : 2.0) * energy_integrand(p, pinj, q, pmax);
+        }
+        sums[k] = warp_sum(s);
+    }
+    team.sync();   // part's readers of the tracer before are done
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int k = 0; k < 8 / WARPS; k++) part[k * WARPS + team.warp] = sums[k];
+    }
+    team.sync();
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) s += part[w];
     s += energy_integrand(pinj, pinj, q, pmax) + energy_integrand(pmax, pinj, q, pmax);
     return k4Pi * kMpG * kCExact * kCExact * (s * h / 3.0);
 }
@@ -381,21 +408,26 @@ __device__ double reacc_adiabatic(const DsaArgs &A, int s, const double *N, doub
     return delta_edens(A, s, ad, pmin, lane);
 }
 
-// The shocks of the block's tracers, the reacceleration and adiabatic deltas of
-// both species, the partial sums of the Simpson integral and the species' energy
+// A team's reacceleration and adiabatic deltas of both species (not there without
+// reacceleration); its partial sums of the Simpson integral and the species' energy
 // sums.
-struct DsaSmem {
-    DsaShock shock[kDsaTracers];
+struct DsaRows {
     double dlt[2][NB], ad[2][NB];
-    double part[kDsaThreads / 32];
+};
+struct DsaSums {
+    double part[8];
     double e_dlt[2], e_ad[2], budget;
 };
 
-// All threads of the block on tracer t and its shock k.
-__device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &sm)
+// A team on tracer t and its shock k.
+template <int WARPS>
+__device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaRows *rows, DsaSums *sums)
 {
+    const DsaTeam<WARPS> team;
+    DsaRows &sm = rows[team.index];
+    DsaSums &sum = sums[team.index];
     const CromaB200DsaParams &prm = A.prm;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = team.warp;
     const double mach = k.mach, rho1 = k.rho1, u1 = k.u1, q = k.q, pmin_p = k.pmin_p, pmin_e = k.pmin_e;
     const double chi_e = k.chi_e, mass_g = k.mass_g, vup = k.vup, vdown = k.vdown;
     const int inj_p = prm.inject_species != 2, inj_e = prm.inject_species != 1;
@@ -405,7 +437,7 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
     const double eta = dsa_eta(mach, prm.eta_model_initial);
     if (mach > 1.0 && prm.gamma_gas > 1.0 && prm.chi_p > 0.0 && prm.pmax_p_mc > 0.0 && eta > 0.0 &&
         pmin_p < prm.pmax_p_mc) {
-        const double unit = proton_edens_unit(pmin_p, q, prm.pmax_p_mc, sm.part);
+        const double unit = proton_edens_unit<WARPS>(pmin_p, q, prm.pmax_p_mc, sum.part, team);
         if (unit > 0.0 && rho1 > 0.0 && u1 > 0.0 && k.u2 > 0.0)
             A_p = eta * (0.5 * rho1 * u1 * u1 * u1) / k.u2 / unit;
     }
@@ -423,7 +455,7 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
     // reacceleration deltas of the pre-shock spectra: warp 0 protons, warp 1 electrons
     double scale = 0.0, energy = 0.0;
     const bool reacc = A.reacc == 1 || A.reacc == 2;
-    if (reacc) __syncthreads();   // the rows' readers of the tracer before are done
+    if (reacc) team.sync();   // the rows' readers of the tracer before are done
     if (A.reacc == 1) {
         if (warp < 2) {
             // X_cr = P_cr / P_th with E_cr above xcr_pmin (tracer_dsa_xcr_proton)
@@ -451,22 +483,22 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
             const double budget = extra * 0.5 * mass_g * u1 * u1;
             if (budget > 0.0) {
                 const double es = reacc_positive(A, warp, warp ? Ne : Np, vdown, q, warp ? pmin_e : pmin_p, sm.dlt[warp], lane);
-                if (lane == 0) sm.e_dlt[warp] = es;
+                if (lane == 0) sum.e_dlt[warp] = es;
             }
-            if (threadIdx.x == 0) sm.budget = budget;
+            if (team.tid == 0) sum.budget = budget;
         }
-        __syncthreads();
-        const double budget = sm.budget;
+        team.sync();
+        const double budget = sum.budget;
         bool none = true;
         if (budget > 0.0) {
-            energy = (sm.e_dlt[0] + sm.e_dlt[1]) * vdown;
+            energy = (sum.e_dlt[0] + sum.e_dlt[1]) * vdown;
             if (energy > 0.0 && isfinite(energy)) {
                 scale = (energy > budget) ? budget / energy : 1.0;
                 none = false;
             }
         }
         if (none) {   // each thread the bins that it applies below
-            for (int j = threadIdx.x; j < NB; j += kDsaThreads) {
+            for (int j = team.tid; j < NB; j += team.kThreads) {
                 sm.dlt[0][j] = 0.0;
                 sm.dlt[1][j] = 0.0;
             }
@@ -482,28 +514,28 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
             double as = 0.0;
             if (capped) as = reacc_adiabatic(A, warp, N, vup, vdown, k.ratio, pmin, sm.ad[warp], lane);
             if (lane == 0) {
-                sm.e_dlt[warp] = cs;
-                sm.e_ad[warp] = as;
+                sum.e_dlt[warp] = cs;
+                sum.e_ad[warp] = as;
             }
         }
-        __syncthreads();
-        const double cp = sm.e_dlt[0], ce = sm.e_dlt[1];
+        team.sync();
+        const double cp = sum.e_dlt[0], ce = sum.e_dlt[1];
         energy = (cp + ce) * vdown;
         scale = 1.0;
         if (capped) {
             const double budget = prm.reacc_eta_cap * 0.5 * mass_g * u1 * u1;
-            const double ap = sm.e_ad[0], ae = sm.e_ad[1];
+            const double ap = sum.e_ad[0], ae = sum.e_ad[1];
             const double nonad = (cp + ce - ap - ae) * vdown;
             if (nonad > 0.0 && isfinite(nonad) && budget > 0.0 && isfinite(budget)) {
                 if (nonad > budget) scale = budget / nonad;
-                for (int j = threadIdx.x; j < NB; j += kDsaThreads) {   // each thread the bins that it applies below
+                for (int j = team.tid; j < NB; j += team.kThreads) {   // each thread the bins that it applies below
                     sm.dlt[0][j] = sm.ad[0][j] + scale * (sm.dlt[0][j] - sm.ad[0][j]);
                     sm.dlt[1][j] = sm.ad[1][j] + scale * (sm.dlt[1][j] - sm.ad[1][j]);
                 }
                 energy = (ap + ae + scale * (cp + ce - ap - ae)) * vdown;
             }
         }
-        if (A.dis && threadIdx.x == 0) A.dis[t] = 1;
+        if (A.dis && team.tid == 0) A.dis[t] = 1;
     }
 
     // apply: fresh sources, then the reacceleration deltas (from the
@@ -514,7 +546,7 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
     const double inv_dt = state ? 1.0 : 1.0 / A.dt_gyr;
     const double s_re = (A.reacc == 2) ? 1.0 : scale;
     const double *gp = A.dsa_p, *ge = A.dsa_p + NB;
-    for (int j = threadIdx.x; j < NB; j += kDsaThreads) {
+    for (int j = team.tid; j < NB; j += team.kThreads) {
         double vp = Op[j * A.js], ve = Oe[j * A.js];
         if (inj_p && fresh_p) {
             const double src = source_dp(A_p, pmin_p, q, prm.pmax_p_mc, gp[j]);
@@ -533,24 +565,36 @@ __device__ void dsa_tracer(const DsaArgs &A, int t, const DsaShock &k, DsaSmem &
     }
     bool applied = (inj_p && fresh_p) || (inj_e && fresh_p && fresh_e);
     if (reacc && scale > 0.0 && isfinite(energy) && fabs(energy) > 0.0) applied = true;
-    if (applied && threadIdx.x == 0) atomicAdd(A.count, 1u);
+    if (applied && team.tid == 0) atomicAdd(A.count, 1u);
 }
 
 __global__ void __launch_bounds__(kDsaThreads, 3) dsa_inject_kernel(const __grid_constant__ DsaArgs A)
 {
-    __shared__ DsaSmem sm;
+    extern __shared__ double4 dsa_smem[];
+    __shared__ DsaShock shock[kDsaTracers];
+    __shared__ DsaSums sums[4];
     __shared__ unsigned shocked;
+    DsaRows *rows = reinterpret_cast<DsaRows *>(dsa_smem);
     const int t0 = blockIdx.x * A.per_block;
     if (threadIdx.x < 32) {
         const int t = t0 + threadIdx.x;
-        const bool hit = threadIdx.x < A.per_block && t < A.ntracer && dsa_shock(A, t, sm.shock[threadIdx.x & (kDsaTracers - 1)]);
+        const bool hit = threadIdx.x < A.per_block && t < A.ntracer && dsa_shock(A, t, shock[threadIdx.x & (kDsaTracers - 1)]);
         const unsigned m = __ballot_sync(kFull, hit);
         if (threadIdx.x == 0) shocked = m;
     }
     __syncthreads();
-    for (unsigned m = shocked; m; m &= m - 1) {
-        const int i = __ffs(m) - 1;
-        dsa_tracer(A, t0 + i, sm.shock[i], sm);
+    if (__popc(shocked) < (A.reacc ? kDsaPairsReacc : kDsaPairs)) {
+        for (unsigned m = shocked; m; m &= m - 1) {
+            const int i = __ffs(m) - 1;
+            dsa_tracer<8>(A, t0 + i, shock[i], rows, sums);
+        }
+    } else {
+        const int team = threadIdx.x / 64;
+        int k = 0;
+        for (unsigned m = shocked; m; m &= m - 1, k++) {
+            const int i = __ffs(m) - 1;
+            if ((k & 3) == team) dsa_tracer<2>(A, t0 + i, shock[i], rows, sums);
+        }
     }
 }
 
@@ -630,7 +674,11 @@ int dsa_inject(Context &c, const CromaB200Shocks *sh, double density_unit, doubl
     }
     CROMA_CUDA(cudaMemsetAsync(c.d_dis, 0, (size_t)n, c.stream));
     CROMA_CUDA(cudaMemsetAsync(c.d_dsa_count, 0, sizeof(unsigned), c.stream));
-    dsa_inject_kernel<<<(n + A.per_block - 1) / A.per_block, kDsaThreads, 0, c.stream>>>(A);
+    // no rows without reacceleration, one team's where a block can have no more, else four teams'
+    const size_t smem = (A.reacc == 0 ? 0 : (A.per_block < kDsaPairsReacc ? 1 : 4)) * sizeof(DsaRows);
+    static OncePerDevice once;
+    CROMA_CUDA(allow_smem(once, dsa_inject_kernel, 4 * sizeof(DsaRows)));
+    dsa_inject_kernel<<<(n + A.per_block - 1) / A.per_block, kDsaThreads, smem, c.stream>>>(A);
     CROMA_CUDA(cudaGetLastError());
     c.last_launches += 1;
     unsigned cnt = 0;
