@@ -261,7 +261,7 @@ def run_resident(path, cfg, nt, w, bg_dev, sh_dev, snaps, warmup, steps, emissio
                 emis_events.append((e0, e1))
             # the GEMMs (one launch), the IC table and its weights (z changes every snapshot),
             # the synchrotron plane keys, the radix sort's 4 kernels, the synchrotron
-            launches += 10
+            launches += 9
         fp.snapshot(bg_dev[k].data_ptr(), bg_dev[k + 1].data_ptr(), float(w.z[isnap]), float(w.z[isnap + 1]),
                     True, float(w.dt[isnap]), float(w.elapsed[isnap]), sync=False)
         launches += fp.last_launch_count()

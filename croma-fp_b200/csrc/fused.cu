@@ -398,10 +398,11 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 // Measured, before (a warp per system at every bin count, coefficients staged
 // in shared memory, a reciprocal a row in the serial chain of the pivots) and
 // now, protons and electrons: 512 bins, 131,072 tracers x 16 segments 20.6 and
-// 16.7 -> 11.2 and 9.0 ms; 256 bins, 65,536 tracers 3.82 and 3.18 -> 2.93 and
-// 2.25 ms; 128 bins, 131,072 tracers (electrons) 3.53 -> 2.25 ms; 64 tracers 61
-// -> 13 us.  12 warps with the rows in registers 12.5 and 11.2 ms at 512 bins,
-// the face loop unrolled whole 12.4 and 9.9.  FP64 pipe 45 %.
+// 16.7 -> 11.0 and 8.8 ms; 256 bins, 65,536 tracers 3.82 and 3.18 -> 2.83 and
+// 2.18 ms; 128 bins, 131,072 tracers (electrons) 3.53 -> 2.18 ms; 64 tracers 61
+// -> 10 us.  12 warps with the rows in registers 12.5 and 11.2 ms at 512 bins,
+// the face loop unrolled whole 12.4 and 9.9.  FP64 pipe 46 and 42 % (512 bins,
+// 4,096 tracers).
 // Tables are pairs of doubles, read 16 bytes at a time:
 enum { FT_X01,      // electrons: p^2, 1/beta^2;  protons: 1/beta^2, that / (2 m_p (gamma - 1))
        FT_X2P,      // electrons: log p / beta^2, p;  protons: sig_eff, p
@@ -1633,13 +1634,16 @@ __global__ void __launch_bounds__(WPB * 32,
 //   present one: all warps of an SM keep step, and would ask for 190 KB at once.
 //
 // All terms are nonnegative (an M-matrix, nonnegative spectra), so nothing
-// cancels and the error is the two-pass form's.
+// cancels.  A row is rounded five times a sub-step where the two-pass form rounds
+// three times: after 500 sub-steps the mean 2-norm error against 80 bits is 1.04
+// of that form's with the same factors (3e-15; the largest element's, 1e-12 at
+// the spectra's far ends, is the coefficients' and the same).
 //
 // Measured, whole kernel with its segment switches, before (a warp per tracer)
 // and now: 131,072 tracers x 500 sub-steps of 128 bins 8.20 -> 4.42 ms, of 512
-// bins 24.6 -> 20.6 ms (with a source 25.4 -> 21.3), 65,536 of 256 bins 6.24 ->
+// bins 24.6 -> 20.8 ms (with a source 25.4 -> 21.0), 65,536 of 256 bins 6.24 ->
 // 5.2 ms; 30,011 with 11 to 500 sub-steps 0.60 -> 0.25 ms; 64 tracers 152 ->
-// 131 us.  FP64 pipe 52 % (its operand reads ~70 %), stalls per issue:
+// 130 us.  FP64 pipe 49 % at 512 bins and 4,096 tracers, stalls per issue:
 // dependent FP64 1.9, shuffles and tensor memory 0.7 to 1.2.
 constexpr int kPkWarps = 4;               // one per TMEM lane quarter
 constexpr int kPkColumns = 128;           // TMEM columns of a block: 3 blocks per SM hold 384 of 512
@@ -2189,8 +2193,8 @@ cudaError_t launch_order(cudaStream_t st, int nt, const int *nsub, unsigned *bin
 // 40 of 64 bits a sub-step) and their latency bound it.  Before (each lane
 // loading its rows, half a cache line apart, as the sub-step began; the source
 // and all scan multipliers in registers) and now, both species, 512 bins 58.1 ->
-// 40.0 ms a snapshot of 16,384 tracers and 3.06 -> 2.78 ms of 64, 256 bins 19.8
-// -> 18.3 and 2.28 -> 2.07, 128 bins 11.3 -> 11.1 and 1.91 -> 1.70.  Sixteen
+// 41.0 ms a snapshot of 16,384 tracers and 3.06 -> 2.98 ms of 64, 256 bins 19.8
+// -> 18.3 and 2.28 -> 2.09, 128 bins 11.3 -> 11.0 and 1.91 -> 1.62.  Sixteen
 // rows a lane and two or four systems a warp, with half the shuffles, took 22.0
 // and 11.5 ms at 256 and 128 bins: too few warps for the longer chains.
 constexpr int kPlainBlocks = NB <= 128 ? 24 : (NB <= 256 ? 20 : 12);   // per SM
